@@ -36,6 +36,7 @@
 
 #include "shl_geom.h"
 #include "shl_internal.cuh"
+#include "shl_pairs.cuh"
 
 namespace shl {
 
@@ -738,9 +739,14 @@ __device__ __forceinline__ void narrow_accept(const DevBuf& b, const StepConst& 
 __global__ void __launch_bounds__(kBlock) k_rb_narrow(DevBuf b, StepConst sc) {
   Ctl* ctl = b.ctl;
   if (rb_off(ctl)) return;
+  extern __shared__ __align__(16) unsigned char pair_smem[];
+  PairWork& work = *reinterpret_cast<PairWork*>(pair_smem);
   const uint32_t n = min(ctl->n_cand, sc.cand_cap);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t e1 = b.cand_e1[i], e2 = b.cand_e2[i];
+  for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+    const uint32_t i = i0 + threadIdx.x;
+    const bool active = i < n;
+    const uint32_t ii = active ? i : i0;
+    const uint32_t e1 = b.cand_e1[ii], e2 = b.cand_e2[ii];
     const double* P1[3];
     const double* P2[3];
     for (int q = 0; q < 3; ++q) {
@@ -748,8 +754,8 @@ __global__ void __launch_bounds__(kBlock) k_rb_narrow(DevBuf b, StepConst sc) {
       P2[q] = b.p + 3 * (size_t)b.tri[3 * (size_t)e2 + q];
     }
     shl_pair_geom g;
-    shl_pair_compute(P1, P2, &g);
-    narrow_accept(b, sc, ctl, i, e1, g.d2);
+    pair_compute_block(active, P1, P2, work, &g);
+    if (active) narrow_accept(b, sc, ctl, i, e1, g.d2);
   }
 }
 
@@ -1263,9 +1269,12 @@ void launch_smooth_search(const DevBuf& b, const StepConst& sc, bool rebuild, cu
     k_smooth_search<false><<<search_grid<false>(), kSearchBlock, 0, s>>>(b, sc);
 }
 
-// k_csr_sort_big takes more than the default 48 KB of shared memory; called
+// k_csr_sort_big and k_rb_narrow take more than the default 48 KB of shared memory; called
 // once per device before its first launch
 cudaError_t init_contact_kernels() {
+  const cudaError_t e = cudaFuncSetAttribute((const void*)k_rb_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(PairWork));
+  if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute((const void*)k_csr_sort_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(kCsrSortBigCap * 4));
 }
@@ -1318,7 +1327,7 @@ void launch_rebuild(const DevBuf& b, const StepConst& sc, cudaStream_t s) {
     if (sc.smooth)
       launch_smooth_search(b, sc, true, s);
     else
-      k_rb_narrow<<<gc, kBlock, 0, s>>>(b, sc);
+      k_rb_narrow<<<gc, kBlock, sizeof(PairWork), s>>>(b, sc);
     launch_scan(&b.ctl->rebuild, b.ctl, b.new_cnt, b.new_off, nullptr, sc.F, sc.F, b.scan_block, &b.ctl->n_new,
                 false, sc.pairs_cap, true, s);
     k_rb_scatter_new<<<gc, kBlock, 0, s>>>(b, sc);

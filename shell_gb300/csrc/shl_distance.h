@@ -105,14 +105,14 @@ SHL_HD void shl_segment_segment(const double* p10, const double* p11,
       /* parallel segments: any s works, take the start of segment 1 */
       s = denom > 0.0 ? shl_clamp01(SHL_DIV(SHL_SUB(SHL_MUL(b, f), SHL_MUL(c, e)), denom)) : 0.0;
       const double tnom = SHL_ADD(SHL_MUL(b, s), f);
-      if (tnom < 0.0) {
-        t = 0.0;
-        s = shl_clamp01(SHL_DIV(-c, a));
-      } else if (tnom > e) {
-        t = 1.0;
-        s = shl_clamp01(SHL_DIV(SHL_SUB(b, c), a));
+      /* one division for the three ranges of t (a warp's lanes take all of them) */
+      const int low = tnom < 0.0, high = tnom > e;
+      const double q = SHL_DIV(low ? -c : (high ? SHL_SUB(b, c) : tnom), low || high ? a : e);
+      if (low || high) {
+        t = low ? 0.0 : 1.0;
+        s = shl_clamp01(q);
       } else {
-        t = SHL_DIV(tnom, e);
+        t = q;
       }
     }
   }
@@ -145,25 +145,34 @@ SHL_HD void shl_point_triangle(const double* p0, const double* p1, const double*
   const double vc = SHL_SUB(SHL_MUL(d1, d4), SHL_MUL(d3, d2));
   const double vb = SHL_SUB(SHL_MUL(d5, d2), SHL_MUL(d1, d6));
   const double va = SHL_SUB(SHL_MUL(d3, d6), SHL_MUL(d5, d4));
-  if (d1 <= 0.0 && d2 <= 0.0) {            /* vertex p1 */
-    v = 0.0; w = 0.0;
-  } else if (d3 >= 0.0 && d4 <= d3) {      /* vertex p2 */
-    v = 1.0; w = 0.0;
-  } else if (vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0) {  /* edge p1-p2 */
-    v = SHL_DIV(d1, SHL_SUB(d1, d3)); w = 0.0;
-  } else if (d6 >= 0.0 && d5 <= d6) {      /* vertex p3 */
-    v = 0.0; w = 1.0;
-  } else if (vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0) {  /* edge p1-p3 */
-    v = 0.0; w = SHL_DIV(d2, SHL_SUB(d2, d6));
-  } else if (va <= 0.0 && SHL_SUB(d4, d3) >= 0.0 && SHL_SUB(d5, d6) >= 0.0) {  /* edge p2-p3 */
-    const double e43 = SHL_SUB(d4, d3);
-    w = SHL_DIV(e43, SHL_ADD(e43, SHL_SUB(d5, d6)));
-    v = SHL_SUB(1.0, w);
-  } else {                                 /* interior */
-    const double den = SHL_ADD(SHL_ADD(va, vb), vc);
-    v = SHL_DIV(vb, den);
-    w = SHL_DIV(vc, den);
+  /* the region, and the quotient that it needs: one division for all of them
+   * (a warp's lanes lie in different regions), a second one for the interior */
+  double num = 0.0, den = 1.0;
+  int region;                              /* 0-2 vertex p1-p3, 3 p1-p2, 4 p1-p3, 5 p2-p3, 6 interior */
+  if (d1 <= 0.0 && d2 <= 0.0) {
+    region = 0;
+  } else if (d3 >= 0.0 && d4 <= d3) {
+    region = 1;
+  } else if (vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0) {
+    region = 3;
+    num = d1; den = SHL_SUB(d1, d3);
+  } else if (d6 >= 0.0 && d5 <= d6) {
+    region = 2;
+  } else if (vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0) {
+    region = 4;
+    num = d2; den = SHL_SUB(d2, d6);
+  } else if (va <= 0.0 && SHL_SUB(d4, d3) >= 0.0 && SHL_SUB(d5, d6) >= 0.0) {
+    region = 5;
+    num = SHL_SUB(d4, d3); den = SHL_ADD(num, SHL_SUB(d5, d6));
+  } else {
+    region = 6;
+    num = vb; den = SHL_ADD(SHL_ADD(va, vb), vc);
   }
+  const double qt = SHL_DIV(num, den);
+  v = region == 3 || region == 6 ? qt : (region == 1 ? 1.0 : 0.0);
+  w = region == 4 || region == 5 ? qt : (region == 2 ? 1.0 : 0.0);
+  if (region == 5) v = SHL_SUB(1.0, w);
+  if (region == 6) w = SHL_DIV(vc, den);
   const double u = SHL_SUB(SHL_SUB(1.0, v), w);
   double q[3];
   for (int k = 0; k < 3; ++k)

@@ -35,51 +35,74 @@ typedef struct shl_pair_geom {
   double v[2], w[2];  /* barycentric coordinates on elements 1 and 2 */
 } shl_pair_geom;
 
-/* p1[k], p2[k]: vertex k of element 1 / element 2 (3 doubles each). */
-SHL_HD void shl_pair_compute(const double* const* p1, const double* const* p2, shl_pair_geom* g)
+/* Edge i of element 1 against edge j of element 2, edge k running from node k
+ * to node (k+1)%3: takes the test's result into g if it is below g->d2. */
+SHL_HD void shl_pair_take_edges(int i, int j, double d2, const double* dc, const double* st, shl_pair_geom* g)
+{
+  if (d2 < g->d2) {
+    g->d2 = d2;
+    g->dc[0] = dc[0]; g->dc[1] = dc[1]; g->dc[2] = dc[2];
+    const double s0 = st[0], s1 = st[1];
+    g->v[0] = (i == 0) ? s0 : ((i == 1) ? SHL_SUB(1.0, s0) : 0.0);
+    g->w[0] = (i == 1) ? s0 : ((i == 2) ? SHL_SUB(1.0, s0) : 0.0);
+    g->v[1] = (j == 0) ? s1 : ((j == 1) ? SHL_SUB(1.0, s1) : 0.0);
+    g->w[1] = (j == 1) ? s1 : ((j == 2) ? SHL_SUB(1.0, s1) : 0.0);
+  }
+}
+
+/* Vertex j of element i + 1 against the other element's face. */
+SHL_HD void shl_pair_take_vertex(int i, int j, double d2, const double* dc, const double* vw, shl_pair_geom* g)
+{
+  if (d2 < g->d2) {
+    g->d2 = d2;
+    if (i == 0) { g->dc[0] = dc[0]; g->dc[1] = dc[1]; g->dc[2] = dc[2]; }
+    else { g->dc[0] = -dc[0]; g->dc[1] = -dc[1]; g->dc[2] = -dc[2]; }
+    const double jv = (j == 1) ? 1.0 : 0.0, jw = (j == 2) ? 1.0 : 0.0;
+    g->v[0] = (i == 0) ? jv : vw[0];
+    g->w[0] = (i == 0) ? jw : vw[1];
+    g->v[1] = (i == 1) ? jv : vw[0];
+    g->w[1] = (i == 1) ? jw : vw[1];
+  }
+}
+
+SHL_HD void shl_pair_none(shl_pair_geom* g)
 {
   g->d2 = SHL_DBL_MAX;
   g->dc[0] = g->dc[1] = g->dc[2] = 0.0;
   g->v[0] = g->v[1] = g->w[0] = g->w[1] = 0.0;
-  /* edge-edge: edge i of element 1 runs from node i to node (i+1)%3 */
+}
+
+/* p1[k], p2[k]: vertex k of element 1 / element 2 (3 doubles each); the tests
+ * of `mask` (bit 3 i + j edges, bit 9 + 3 i + j vertex) in their fixed order. */
+SHL_HD void shl_pair_compute_masked(const double* const* p1, const double* const* p2, unsigned mask, shl_pair_geom* g)
+{
+  shl_pair_none(g);
   for (int i = 0; i < 3; ++i) {
     const int i1 = (i == 2) ? 0 : i + 1;
     for (int j = 0; j < 3; ++j) {
+      if (!((mask >> (3 * i + j)) & 1u)) continue;
       const int j1 = (j == 2) ? 0 : j + 1;
       double dc[3], st[2];
       shl_segment_segment(p1[i], p1[i1], p2[j], p2[j1], dc, st);
-      const double d2 = shl_v3_dot(dc, dc);
-      if (d2 < g->d2) {
-        g->d2 = d2;
-        g->dc[0] = dc[0]; g->dc[1] = dc[1]; g->dc[2] = dc[2];
-        const double s0 = st[0], s1 = st[1];
-        g->v[0] = (i == 0) ? s0 : ((i == 1) ? SHL_SUB(1.0, s0) : 0.0);
-        g->w[0] = (i == 1) ? s0 : ((i == 2) ? SHL_SUB(1.0, s0) : 0.0);
-        g->v[1] = (j == 0) ? s1 : ((j == 1) ? SHL_SUB(1.0, s1) : 0.0);
-        g->w[1] = (j == 1) ? s1 : ((j == 2) ? SHL_SUB(1.0, s1) : 0.0);
-      }
+      shl_pair_take_edges(i, j, shl_v3_dot(dc, dc), dc, st, g);
     }
   }
-  /* vertex-face: vertex j of one element against the face of the other */
   for (int i = 0; i < 2; ++i) {
     const double* const* pv = (i == 0) ? p1 : p2;
     const double* const* pf = (i == 0) ? p2 : p1;
     for (int j = 0; j < 3; ++j) {
+      if (!((mask >> (9 + 3 * i + j)) & 1u)) continue;
       double dc[3], vw[2];
       shl_point_triangle(pv[j], pf[0], pf[1], pf[2], dc, vw);
-      const double d2 = shl_v3_dot(dc, dc);
-      if (d2 < g->d2) {
-        g->d2 = d2;
-        if (i == 0) { g->dc[0] = dc[0]; g->dc[1] = dc[1]; g->dc[2] = dc[2]; }
-        else { g->dc[0] = -dc[0]; g->dc[1] = -dc[1]; g->dc[2] = -dc[2]; }
-        const double jv = (j == 1) ? 1.0 : 0.0, jw = (j == 2) ? 1.0 : 0.0;
-        g->v[0] = (i == 0) ? jv : vw[0];
-        g->w[0] = (i == 0) ? jw : vw[1];
-        g->v[1] = (i == 1) ? jv : vw[0];
-        g->w[1] = (i == 1) ? jw : vw[1];
-      }
+      shl_pair_take_vertex(i, j, shl_v3_dot(dc, dc), dc, vw, g);
     }
   }
+}
+
+/* all fifteen tests */
+SHL_HD void shl_pair_compute(const double* const* p1, const double* const* p2, shl_pair_geom* g)
+{
+  shl_pair_compute_masked(p1, p2, 0x7fffu, g);
 }
 
 /* ---- Margolis slip-stick friction, Friction.C:4-60 ------------------------ */

@@ -26,6 +26,7 @@
 #include "shl_geom.h"
 #include "shl_internal.cuh"
 #include "shl_df.cuh"
+#include "shl_pairs.cuh"
 
 namespace shl {
 
@@ -1587,9 +1588,16 @@ __global__ void __launch_bounds__(kBlock) k_contact_force(DevBuf b, StepConst sc
     }
     return;
   }
+  extern __shared__ __align__(16) unsigned char pair_smem[];
+  PairWork& work = *reinterpret_cast<PairWork*>(pair_smem);  // LINEAR
+  static_assert(kPairBlock == kBlock, "pair_compute_block runs on the kernel's blocks");
   double eself = 0.0, efric = 0.0, nc = 0.0;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n_pairs; j += gridDim.x * blockDim.x) {
-    const uint32_t e[2] = {b.pe1[0][j], b.pe2[0][j]};
+  // whole blocks step through the list together (pair_compute_block)
+  for (uint32_t j0 = blockIdx.x * blockDim.x; j0 < n_pairs; j0 += gridDim.x * blockDim.x) {
+    const uint32_t j = j0 + threadIdx.x;
+    const bool active = j < n_pairs;
+    const uint32_t jj = active ? j : j0;
+    const uint32_t e[2] = {b.pe1[0][jj], b.pe2[0][jj]};
     // the shell's contact constants (a pair of a batch lies within one shell)
     const ShellCell* S = sc.n_cs ? &b.shc[b.face_shell[e[0]]] : nullptr;
     const double h = S ? S->thickness : sc.thickness;
@@ -1608,16 +1616,17 @@ __global__ void __launch_bounds__(kBlock) k_contact_force(DevBuf b, StepConst sc
     }
     shl_pair_geom g;
     double* out = b.pforce + kPairOut * (size_t)j;
-    if (SMOOTH) {  // SmoothShellShellContact::compute: the search of k_smooth_search from the previous solution
+    if (SMOOTH && active) {  // SmoothShellShellContact::compute: the search of k_smooth_search from the previous solution
       double x[4];
       for (int k = 0; k < 4; ++k) x[k] = b.pvw[0][4 * (size_t)j + k];
       g.d2 = b.pd2[0][j];
       for (int c = 0; c < 3; ++c) g.dc[c] = out[c];
       smooth_coords(b, e[0], e[1], x, &g);
-    } else {
-      shl_pair_compute(P1, P2, &g);
-      b.pd2[0][j] = g.d2;
+    } else if (!SMOOTH) {
+      pair_compute_block(active, P1, P2, work, &g);
+      if (active) b.pd2[0][j] = g.d2;
     }
+    if (!active) continue;  // past the list's end: no further trip either
     if (g.d2 <= 0.0) register_problem(ctl, SHL_CONTACT_PROBLEM);
     if (g.d2 < d2_friction) {
       const double area_min = fmin(b.area[e[0]], b.area[e[1]]);
@@ -2336,6 +2345,9 @@ cudaError_t init_element_kernels() {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   };
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)k_contact_force<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(PairWork));
   set((const void*)k_elements_df<256, 1>, 256);
   set((const void*)k_elements_df<128, 3>, 128);
   set((const void*)k_elements_df<64, 6>, 64);
@@ -2378,7 +2390,7 @@ void launch_contact_force(const DevBuf& b, const StepConst& sc, int, cudaStream_
     launch_smooth_search(b, sc, false, s);
     k_contact_force<true><<<nb, kBlock, 0, s>>>(b, sc);
   } else
-    k_contact_force<false><<<nb, kBlock, 0, s>>>(b, sc);
+    k_contact_force<false><<<nb, kBlock, sizeof(PairWork), s>>>(b, sc);
 }
 // mode 2: an adaptive attempt (a_pred and the error estimate); else correct ? step corrector : evaluation
 void launch_gather_correct(const DevBuf& b, const StepConst& sc, int mode, bool correct, double* f_out, double* a_out,
