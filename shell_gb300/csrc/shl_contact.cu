@@ -1135,13 +1135,13 @@ __global__ void k_csr_fill(DevBuf b, StepConst sc) {
   }
 }
 
-// sort each node's entries (deterministic order for the gather): a bitonic
-// sort of the entries padded to a power of two in shared memory, by one warp
-// for a node of up to kCsrSortCap entries (a few hundred in a contact-heavy
-// state, about a thousand with SMOOTH contact), by a block of k_csr_sort_big
-// up to kCsrSortBigCap, in place by one thread beyond
+// Sort each node's entries (deterministic order for the gather): by one warp in
+// registers up to kCsrSortCap entries (a few hundred in a contact-heavy state, up
+// to about a thousand with SMOOTH contact), by a block of k_csr_sort_big in
+// shared memory up to kCsrSortBigCap, in place by one thread beyond.
 constexpr int kCsrSortWarps = 4;
-constexpr uint32_t kCsrSortCap = 2048;
+constexpr int kCsrSortNodes = 8;  // nodes per warp
+constexpr uint32_t kCsrSortCap = 1024;
 constexpr uint32_t kCsrSortBigCap = 16384;
 constexpr int kCsrSortBigBlock = 1024;
 
@@ -1193,47 +1193,73 @@ __global__ void __launch_bounds__(kCsrSortBigBlock) k_csr_sort_big(DevBuf b, Ste
   }
 }
 
+// Bitonic sort of n <= 32 E entries by one warp, in registers: element
+// lane * E + r lies in register r of its lane, so the network's strides below E
+// compare registers of one lane and the larger ones take one shuffle each.
+template <int E>
+__device__ __forceinline__ void warp_sort_segment(uint32_t* ent, uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t x[E];
+#pragma unroll
+  for (int r = 0; r < E; ++r) x[r] = (uint32_t)r * 32u + lane < n ? ent[(uint32_t)r * 32u + lane] : 0xffffffffu;
+  __syncwarp();
+#pragma unroll
+  for (int k = 2; k <= 32 * E; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j < E) {
+#pragma unroll
+        for (int r = 0; r < E; ++r) {
+          if (r & j) continue;
+          const bool up = k < E ? (r & k) == 0 : (lane & (uint32_t)(k / E)) == 0;
+          const uint32_t lo = min(x[r], x[r | j]), hi = max(x[r], x[r | j]);
+          x[r] = up ? lo : hi;
+          x[r | j] = up ? hi : lo;
+        }
+      } else {
+        const bool up = (lane & (uint32_t)(k / E)) == 0, first = (lane & (uint32_t)(j / E)) == 0;
+#pragma unroll
+        for (int r = 0; r < E; ++r) {
+          const uint32_t y = __shfl_xor_sync(0xffffffffu, x[r], j / E);
+          x[r] = up == first ? min(x[r], y) : max(x[r], y);
+        }
+      }
+    }
+#pragma unroll
+  for (int r = 0; r < E; ++r)
+    if (lane * E + r < n) ent[lane * E + r] = x[r];
+  __syncwarp();
+}
+
+// One warp takes kCsrSortNodes consecutive nodes.  The sort is a chain of
+// dependent compares, so it wants many warps and no shared memory: in shared
+// memory, with 32 nodes per warp (8 warps per SM), a folded level-6 shell (41 k
+// nodes, 250 entries each) took 1.37 ms, now 0.1; with SMOOTH contact (level 5, 630
+// each) 2.15 ms, now 0.14 and 0.09 in k_csr_sort_big.
 __global__ void __launch_bounds__(32 * kCsrSortWarps) k_csr_sort(DevBuf b, StepConst sc) {
   Ctl* ctl = b.ctl;
   if (csr_off(ctl)) return;
-  __shared__ uint32_t buf[kCsrSortWarps][kCsrSortCap];
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  uint32_t* sh = buf[w];
-  // each warp reads the segments of 32 consecutive nodes at once and sorts the
-  // ones with two or more entries; larger ones than the buffer go to the list
-  for (uint32_t base = (blockIdx.x * kCsrSortWarps + w) * 32; base < sc.V; base += gridDim.x * kCsrSortWarps * 32) {
-    const uint32_t me = base + lane;
-    uint32_t k0 = 0, n = 0;
-    if (me < sc.V) {
-      k0 = b.csr_ptr[me];
-      n = b.csr_ptr[me + 1] - k0;
-    }
-    if (n > kCsrSortCap) b.csr_fill[atomicAdd(&ctl->cnt[9], 1u)] = me;
-    unsigned todo = __ballot_sync(0xffffffffu, n >= 2 && n <= kCsrSortCap);
-    while (todo) {
-      const int src = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint32_t s0 = __shfl_sync(0xffffffffu, k0, src), sn = __shfl_sync(0xffffffffu, n, src);
-      uint32_t P = 32;
-      while (P < sn) P <<= 1;
-      for (uint32_t i = lane; i < P; i += 32) sh[i] = i < sn ? b.csr_ent[s0 + i] : 0xffffffffu;
-      __syncwarp();
-      for (uint32_t k = 2; k <= P; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-          // compare-exchange t: the pair (i, i + j) with bit j of i clear
-          for (uint32_t t = lane; t < P / 2; t += 32) {
-            const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1));
-            const uint32_t x = sh[i], y = sh[i + j];
-            if (((i & k) == 0) == (x > y)) {
-              sh[i] = y;
-              sh[i + j] = x;
-            }
-          }
-          __syncwarp();
-        }
-      for (uint32_t i = lane; i < sn; i += 32) b.csr_ent[s0 + i] = sh[i];
-      __syncwarp();
-    }
+  const uint32_t me = (blockIdx.x * kCsrSortWarps + w) * kCsrSortNodes + lane;
+  uint32_t k0 = 0, n = 0;
+  if (lane < kCsrSortNodes && me < sc.V) {
+    k0 = b.csr_ptr[me];
+    n = b.csr_ptr[me + 1] - k0;
+  }
+  // larger segments than the registers hold go to the list of k_csr_sort_big
+  if (n > kCsrSortCap) b.csr_fill[atomicAdd(&ctl->cnt[9], 1u)] = me;
+  unsigned todo = __ballot_sync(0xffffffffu, n >= 2 && n <= kCsrSortCap);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    uint32_t* ent = b.csr_ent + __shfl_sync(0xffffffffu, k0, src);
+    const uint32_t sn = __shfl_sync(0xffffffffu, n, src);
+    if (sn <= 32) warp_sort_segment<1>(ent, sn);
+    else if (sn <= 64) warp_sort_segment<2>(ent, sn);
+    else if (sn <= 128) warp_sort_segment<4>(ent, sn);
+    else if (sn <= 256) warp_sort_segment<8>(ent, sn);
+    else if (sn <= 512) warp_sort_segment<16>(ent, sn);
+    else warp_sort_segment<32>(ent, sn);
   }
 }
 
@@ -1289,8 +1315,7 @@ void launch_contact_csr(const DevBuf& b, const StepConst& sc, cudaStream_t s) {
               true, sc.csr_cap, true, s);
   k_csr_fill<<<gP, kBlock, 0, s>>>(b, sc);
   {
-    uint32_t g = (sc.V + 32 * kCsrSortWarps - 1) / (32 * kCsrSortWarps);
-    if (g > 16 * 152) g = 16 * 152;
+    const uint32_t g = (sc.V + kCsrSortNodes * kCsrSortWarps - 1) / (kCsrSortNodes * kCsrSortWarps);
     k_csr_sort<<<g ? g : 1, 32 * kCsrSortWarps, 0, s>>>(b, sc);
     k_csr_sort_big<<<152, kCsrSortBigBlock, kCsrSortBigCap * 4, s>>>(b, sc);
   }
