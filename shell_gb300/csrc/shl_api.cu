@@ -26,6 +26,12 @@ namespace {
 thread_local std::string g_err;
 constexpr uint32_t kGraphSteps = 16;
 constexpr uint32_t kTableCap = 1u << 16;
+// Subdivision levels times irregular faces whose children's power forms are made
+// before each SMOOTH search: all 34 levels of the 60 faces around a sphere's
+// twelve irregular vertices, about 10 us of FP64 work and 2 MB; meshes with more
+// irregular faces keep their first levels (level 1 is three quarters of a patch's
+// parameter area, level 2 three quarters of the rest, and so on) or none.
+constexpr uint32_t kIrregularLevels = 2048;
 
 #define SHL_CUDA_TRY(expr)                                                 \
   do {                                                                     \
@@ -648,6 +654,8 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
   // contact buffers
   const bool contact = params->shell_shell_contact != SHL_CONTACT_NONE;
   const bool smooth = params->shell_shell_contact == SHL_CONTACT_SMOOTH;
+  uint32_t irr_first = F;
+  int32_t irr_levels = SHL_SMOOTH_LEVELS;  // no irregular face: nothing beyond the tables
   uint64_t n_cells0 = 0, entries0 = 0;
   uint32_t n_cells_cap = 1, entries_cap = 1, pairs_cap = 1, csr_cap = 1, cand_cap = 1;
   if (contact) {
@@ -699,6 +707,12 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
       ALLOC(b.pvw[0], 4 * (size_t)pairs_cap); ALLOC(b.pvw[1], 4 * (size_t)pairs_cap);
       ALLOC(b.new_x, 4 * (size_t)pairs_cap); ALLOC(b.cand_x, 4 * (size_t)cand_cap);
       ALLOC(b.lcoef, SHL_LIMIT_NCOEF * (size_t)F);
+      irr_first = S.groups[0].count;
+      const uint32_t n_irr = F - irr_first;
+      if (n_irr) {
+        irr_levels = (int32_t)std::min<uint32_t>(SHL_SMOOTH_LEVELS, kIrregularLevels / n_irr);
+        ALLOC(b.icoef, (size_t)n_irr * irr_levels * 3 * SHL_LIMIT_NCOEF);
+      }
       ALLOC(b.inv_perm, F); ALLOC(b.fsm, F);
     }
     if (batch_contact) {
@@ -825,6 +839,8 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
   sc.cand_cap = cand_cap;
   sc.contact = contact ? 1 : 0;
   sc.smooth = smooth ? 1 : 0;
+  sc.irr_first = irr_first;
+  sc.irr_levels = irr_levels;
   c->var64 = default_var64();
   apply_variant(c);
   for (int k = 0; k < 13; ++k) sc.stab_off[k] = stab_off[k];

@@ -759,12 +759,41 @@ __global__ void __launch_bounds__(kBlock) k_rb_narrow(DevBuf b, StepConst sc) {
   }
 }
 
-// the power form of each regular patch at the current positions (irregular
-// patches are evaluated from their subdivision tables in the search)
+// The power form of each regular patch at the current positions, and of the
+// irregular patches' subdivision children (sc.irr_levels levels, three children
+// each; a thread per child and component).  A search evaluates a patch many
+// times: formed in the search, an irregular patch's control points (12 table rows
+// of N + 6 nodes) and coefficients took about 35 us per evaluation of one lane,
+// and the few pairs next to an irregular vertex held the whole launch.
 __global__ void __launch_bounds__(kBlock) k_limit_coeffs(DevBuf b, StepConst sc, bool rebuild) {
   const Ctl* ctl = b.ctl;
   if (rebuild ? rb_off(ctl) : (ctl->halted != 0 || ctl->paused != 0)) return;
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < sc.F; e += gridDim.x * blockDim.x) {
+  const uint32_t n_irr = (sc.F - sc.irr_first) * (uint32_t)sc.irr_levels * 9u;
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < sc.F + n_irr; t += gridDim.x * blockDim.x) {
+    if (t < n_irr) {
+      const int c = (int)(t % 3u), k = (int)(t / 3u % 3u);
+      const uint32_t q = t / 9u;
+      const int n = 1 + (int)(q % (uint32_t)sc.irr_levels);
+      shl_limit_patch lp;
+      smooth_patch(b, sc, b.perm[sc.irr_first + q / (uint32_t)sc.irr_levels], lp);
+      SHL_TABLE signed char BC[12][15] = SHL_BOX_COEFFS;
+      double P[15];
+#pragma unroll
+      for (int m = 0; m < 15; ++m) P[m] = 0.0;
+#pragma unroll
+      for (int s = 0; s < 12; ++s) {
+        const double Q = shl_limit_child_point(&lp, n, k, s, c);
+#pragma unroll
+        for (int m = 0; m < 15; ++m)
+          if (BC[s][m] != 0) P[m] = SHL_FMA((double)BC[s][m], Q, P[m]);
+      }
+      double* out = b.icoef + SHL_LIMIT_NCOEF * (size_t)(t / 3u) + c;
+      const double twelfth = 1.0 / 12.0;
+#pragma unroll
+      for (int m = 0; m < 15; ++m) out[3 * m] = SHL_MUL(P[m], twelfth);
+      continue;
+    }
+    const uint32_t e = t - n_irr;
     if ((b.fsm[e] & 0xff) != 6) continue;
     shl_limit_patch lp;
     smooth_patch(b, sc, e, lp);
@@ -776,25 +805,48 @@ __global__ void __launch_bounds__(kBlock) k_limit_coeffs(DevBuf b, StepConst sc,
   }
 }
 
-// a patch's limit surface at (v, w): the stored power form of a regular patch
-__device__ __forceinline__ void limit_at(const DevBuf& b, uint32_t e, const shl_limit_patch& lp, double v, double w,
-                                         int order, double out[6][3]) {
-  if (lp.N == 6)
-    shl_limit_poly(reinterpret_cast<const double(*)[3]>(b.lcoef + SHL_LIMIT_NCOEF * (size_t)e), v, w, order, 1.0, out);
-  else
-    shl_limit_eval(&lp, v, w, order, out);
+// a patch's limit surface at (v, w) from the stored power forms; deep: also the
+// levels of an irregular patch beyond them
+template <int ORDER, bool DEEP>
+__device__ __noinline__ void limit_at(const DevBuf& b, const StepConst& sc, uint32_t e, double v, double w, double out[6][3]) {
+  double j1 = 1.0;
+  const double* coef = b.lcoef + SHL_LIMIT_NCOEF * (size_t)e;
+  if ((b.fsm[e] & 0xff) != 6) {
+    int n, k;
+    shl_limit_child(&v, &w, &n, &k, &j1);
+    if (DEEP && n > sc.irr_levels) {
+      shl_limit_patch lp;
+      smooth_patch(b, sc, e, lp);
+      double P[15][3];
+      shl_limit_coeffs_child(&lp, n, k, P);
+      shl_limit_poly(P, v, w, ORDER, j1, out);
+      return;
+    }
+    coef = b.icoef +
+           SHL_LIMIT_NCOEF * ((size_t)((b.inv_perm[e] - sc.irr_first) * (uint32_t)sc.irr_levels + (uint32_t)(n - 1)) * 3 + (size_t)k);
+  }
+  shl_limit_poly(reinterpret_cast<const double(*)[3]>(coef), v, w, ORDER, j1, out);
 }
 
-// SMOOTH closest-point searches with lane refill.  A search takes from one to
-// several hundred limit evaluations (most of a squashed shell's pairs end after
-// one to three, a few run the line search to its limit), so one thread per
-// pair would hold each warp until its longest search ends.  Here each lane
-// runs its search as a resumable state (shl_smooth_state): per trip a warp
-// evaluates one point of both limit patches per lane and advances the
-// searches, and a lane whose search has ended takes the next pair from a queue
-// shared by the grid (ctl->cnt[7]; the last warp to leave resets it), so that
-// the lanes stay busy until the queue is empty.  A search's result does not
-// depend on the lane or the order that runs it.
+// SMOOTH closest-point searches in phase-coherent batches.  A search alternates
+// between the order-2 evaluation of an iterate with its Newton step (about 1200
+// FP64 operations) and the order-0 evaluation of a line-search trial (about 180),
+// and takes from one to several hundred of them.  With one search per lane the
+// lanes of a warp sit in different phases, and every trip pays for both with a
+// third of the lanes busy in each.  Here a warp owns kSearchPool searches, kept
+// in shared memory as resumable states (shl_smooth_state), and per trip runs up
+// to 32 of them that are in the same phase; searches with an irregular patch
+// that may have to subdivide beyond the stored children are a class of their own.  With more searches
+// than lanes there is nearly always a full batch of one class.  A finished
+// search's slot is refilled from a queue shared by the grid (ctl->cnt[7]; the
+// last warp to leave resets it).  A search's result does not depend on the lane
+// or the order that runs it.  Folded level-5 shell, 1.4 M candidates at 5.9
+// Newton iterates each: 100 -> 44 ms for a list build's searches (64 ms from the
+// batches, 51 with the irregular children stored, 44 with the failing shifts of
+// shl_smooth_direction passed over and the evaluation out of line), 8.6 -> 3.1 ms
+// per step.  Pools of 64, 96 and 128 searches and two to four blocks per SM are
+// within 3 %.  What is left is the FP64 pipe (57-80 % busy) and, in the list
+// build, instruction fetches of the divergent Newton step.
 //   REBUILD: the candidates of a linked-cell pass, each from (1/3, 1/3, 1/3,
 //   1/3) as a new SmoothShellShellContact (SmoothShellShellContact.C:9-14),
 //   then k_rb_narrow's acceptance;
@@ -802,70 +854,197 @@ __device__ __forceinline__ void limit_at(const DevBuf& b, uint32_t e, const shl_
 //   dc = p2 - p1 go to pvw, pd2 and the pair's force slots 0-2 for
 //   k_contact_force.
 constexpr int kSearchBlock = 128;
+constexpr int kSearchPool = 64;  // searches per warp (a multiple of 32)
+enum : uint8_t { kSearchEmpty = 0, kSearchNewton = 1, kSearchTrial = 2, kSearchDeep = 3 };
+struct SearchPool {
+  double x[4][kSearchPool], xt[4][kSearchPool], d[4][kSearchPool], p1[3][kSearchPool], p2[3][kSearchPool];
+  double f[kSearchPool], alpha[kSearchPool], gd[kSearchPool], dn[kSearchPool];
+  uint32_t j[kSearchPool], e1[kSearchPool], e2[kSearchPool];
+  uint8_t cls[kSearchPool], trial[kSearchPool], it[kSearchPool], ls[kSearchPool], shifted[kSearchPool],
+      after_accept[kSearchPool];
+  uint8_t batch[32];
+};
+
+// One trip of the pool's slot s, whose next evaluation is a Newton iterate's
+// (phase SHL_SMOOTH_EVAL_FGH) or a trial's (SHL_SMOOTH_EVAL_TRIAL).
+template <bool REBUILD, bool DEEP>
+__device__ __forceinline__ void search_trip(const DevBuf& b, const StepConst& sc, Ctl* ctl, SearchPool& w, uint32_t s,
+                                            int phase) {
+  const uint32_t e1 = w.e1[s], e2 = w.e2[s];
+  shl_smooth_state st;
+  st.phase = phase;
+  st.it = w.it[s];
+  st.after_accept = w.after_accept[s];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) st.x[k] = w.x[k][s];
+  if (phase == SHL_SMOOTH_EVAL_TRIAL) {
+    st.f = w.f[s];
+    st.alpha = w.alpha[s];
+    st.gd = w.gd[s];
+    st.dn = w.dn[s];
+    st.ls = w.ls[s];
+    st.shifted = w.shifted[s];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      st.xt[k] = w.xt[k][s];
+      st.d[k] = w.d[k][s];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      st.p1[c] = w.p1[c][s];
+      st.p2[c] = w.p2[c][s];
+    }
+  }
+  {
+    const double* pt = phase == SHL_SMOOTH_EVAL_FGH ? st.x : st.xt;
+    double ev1[6][3], ev2[6][3];
+    if (phase == SHL_SMOOTH_EVAL_FGH) {
+      limit_at<2, DEEP>(b, sc, e1, pt[0], pt[1], ev1);
+      limit_at<2, DEEP>(b, sc, e2, pt[2], pt[3], ev2);
+    } else {
+      limit_at<0, DEEP>(b, sc, e1, pt[0], pt[1], ev1);
+      limit_at<0, DEEP>(b, sc, e2, pt[2], pt[3], ev2);
+    }
+    shl_smooth_take(&st, ev1, ev2);
+  }
+  if (st.phase == SHL_SMOOTH_DONE) {
+    const uint32_t j = w.j[s];
+    w.cls[s] = kSearchEmpty;
+    if (REBUILD) {
+      for (int k = 0; k < 4; ++k) b.cand_x[4 * (size_t)j + k] = st.x[k];
+      narrow_accept(b, sc, ctl, j, e1, st.f);
+    } else {
+      for (int k = 0; k < 4; ++k) b.pvw[0][4 * (size_t)j + k] = st.x[k];
+      b.pd2[0][j] = st.f;
+      double* out = b.pforce + kPairOut * (size_t)j;
+      for (int c = 0; c < 3; ++c) out[c] = SHL_SUB(st.p2[c], st.p1[c]);
+    }
+    return;
+  }
+  w.it[s] = (uint8_t)st.it;
+  w.after_accept[s] = (uint8_t)st.after_accept;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w.x[k][s] = st.x[k];
+  if (st.phase == SHL_SMOOTH_EVAL_TRIAL) {
+    w.alpha[s] = st.alpha;
+    w.ls[s] = (uint8_t)st.ls;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w.xt[k][s] = st.xt[k];
+    if (phase == SHL_SMOOTH_EVAL_FGH) {
+      w.f[s] = st.f;
+      w.gd[s] = st.gd;
+      w.dn[s] = st.dn;
+      w.shifted[s] = (uint8_t)st.shifted;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w.d[k][s] = st.d[k];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        w.p1[c][s] = st.p1[c];
+        w.p2[c][s] = st.p2[c];
+      }
+    }
+  }
+  const bool trial = st.phase == SHL_SMOOTH_EVAL_TRIAL;
+  w.trial[s] = trial ? 1 : 0;
+  if (!DEEP) w.cls[s] = trial ? kSearchTrial : kSearchNewton;
+}
+
+// trips of the deep class, out of line: they are rare, and their copy of the
+// evaluation would crowd the others out of the instruction cache
 template <bool REBUILD>
-__global__ void __launch_bounds__(kSearchBlock) k_smooth_search(DevBuf b, StepConst sc) {
+__device__ __noinline__ void search_trip_deep(const DevBuf& b, const StepConst& sc, Ctl* ctl, SearchPool& w, uint32_t s) {
+  search_trip<REBUILD, true>(b, sc, ctl, w, s, w.trial[s] ? SHL_SMOOTH_EVAL_TRIAL : SHL_SMOOTH_EVAL_FGH);
+}
+
+template <bool REBUILD>
+__global__ void __launch_bounds__(kSearchBlock, 2) k_smooth_search(DevBuf b, StepConst sc) {
   Ctl* ctl = b.ctl;
   uint32_t* queue = &ctl->cnt[7];
   uint32_t* left = &ctl->cnt[8];
   const bool off = REBUILD ? rb_off(ctl) : (ctl->halted != 0 || ctl->paused != 0);
   const uint32_t n = off ? 0u : (REBUILD ? min(ctl->n_cand, sc.cand_cap) : ctl->n_pairs);
+  extern __shared__ __align__(16) unsigned char search_smem[];
+  SearchPool& w = reinterpret_cast<SearchPool*>(search_smem)[threadIdx.x >> 5];
+  constexpr int R = kSearchPool / 32;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned below = (1u << lane) - 1u;
-  bool busy = false, more = n > 0;
-  uint32_t j = 0, e1 = 0, e2 = 0;
-  shl_limit_patch A, B;
-  shl_smooth_state st;
-  for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !busy);
-    if (more && idle) {
-      const int leader = __ffs(idle) - 1;
-      const uint32_t want = (uint32_t)__popc(idle);
+  bool more = n > 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) w.cls[32 * r + lane] = kSearchEmpty;
+  __syncwarp();
+  while (n > 0) {
+    // slots of each class
+    uint8_t cl[R];
+    unsigned count[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      cl[r] = w.cls[32 * r + lane];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) count[k] += __popc(__ballot_sync(0xffffffffu, cl[r] == k));
+    }
+    if (more && count[kSearchEmpty] >= 16) {
+      // refill the empty slots
       uint32_t base = 0;
-      if ((int)lane == leader) base = atomicAdd(queue, want);
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (!(base + want < n)) more = false;  // the queue is empty for every warp
-      if (!busy) {
+      if (lane == 0) base = atomicAdd(queue, count[kSearchEmpty]);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (!(base + count[kSearchEmpty] < n)) more = false;  // the queue is empty for every warp
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const unsigned idle = __ballot_sync(0xffffffffu, cl[r] == kSearchEmpty);
         const uint32_t i = base + (uint32_t)__popc(idle & below);
-        if (i < n) {
-          busy = true;
-          j = i;
-          double x0[4];
-          if (REBUILD) {
-            e1 = b.cand_e1[i];
-            e2 = b.cand_e2[i];
-            for (int k = 0; k < 4; ++k) x0[k] = 1.0 / 3.0;
-          } else {
-            e1 = b.pe1[0][i];
-            e2 = b.pe2[0][i];
-            for (int k = 0; k < 4; ++k) x0[k] = b.pvw[0][4 * (size_t)i + k];
-          }
-          smooth_patch(b, sc, e1, A);
-          smooth_patch(b, sc, e2, B);
-          shl_smooth_start(&st, x0);
-        }
-      }
-    }
-    if (!__any_sync(0xffffffffu, busy)) break;
-    if (busy) {
-      const double* pt = shl_smooth_point(&st);
-      const int order = shl_smooth_order(&st);
-      double ev1[6][3], ev2[6][3];
-      limit_at(b, e1, A, pt[0], pt[1], order, ev1);
-      limit_at(b, e2, B, pt[2], pt[3], order, ev2);
-      shl_smooth_take(&st, ev1, ev2);
-      if (st.phase == SHL_SMOOTH_DONE) {
-        busy = false;
+        base += (uint32_t)__popc(idle);
+        if (cl[r] != kSearchEmpty || i >= n) continue;
+        const uint32_t s = 32 * r + lane;
+        uint32_t e1, e2;
+        double x0[4];
         if (REBUILD) {
-          for (int k = 0; k < 4; ++k) b.cand_x[4 * (size_t)j + k] = st.x[k];
-          narrow_accept(b, sc, ctl, j, e1, st.f);
+          e1 = b.cand_e1[i];
+          e2 = b.cand_e2[i];
+          for (int k = 0; k < 4; ++k) x0[k] = 1.0 / 3.0;
         } else {
-          for (int k = 0; k < 4; ++k) b.pvw[0][4 * (size_t)j + k] = st.x[k];
-          b.pd2[0][j] = st.f;
-          double* out = b.pforce + kPairOut * (size_t)j;
-          for (int c = 0; c < 3; ++c) out[c] = SHL_SUB(st.p2[c], st.p1[c]);
+          e1 = b.pe1[0][i];
+          e2 = b.pe2[0][i];
+          for (int k = 0; k < 4; ++k) x0[k] = b.pvw[0][4 * (size_t)i + k];
         }
+        shl_smooth_state st;
+        shl_smooth_start(&st, x0);
+        w.j[s] = i;
+        w.e1[s] = e1;
+        w.e2[s] = e2;
+        for (int k = 0; k < 4; ++k) w.x[k][s] = st.x[k];
+        w.it[s] = 0;
+        w.after_accept[s] = 0;
+        w.trial[s] = 0;
+        const bool kept = sc.irr_levels == SHL_SMOOTH_LEVELS || ((b.fsm[e1] & 0xff) == 6 && (b.fsm[e2] & 0xff) == 6);
+        w.cls[s] = kept ? kSearchNewton : kSearchDeep;
       }
+      __syncwarp();
+      continue;
     }
+    // the largest class runs a batch
+    int pick = kSearchNewton;
+    if (count[kSearchTrial] > count[pick]) pick = kSearchTrial;
+    if (count[kSearchDeep] > count[pick]) pick = kSearchDeep;
+    if (count[pick] == 0) break;  // no search left (the queue is empty: an empty pool would have been refilled)
+    uint32_t pos = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const unsigned m = __ballot_sync(0xffffffffu, cl[r] == pick);
+      const uint32_t q = pos + (uint32_t)__popc(m & below);
+      if (cl[r] == pick && q < 32) w.batch[q] = (uint8_t)(32 * r + lane);
+      pos += (uint32_t)__popc(m);
+    }
+    __syncwarp();
+    if (lane < count[pick]) {
+      const uint32_t s = w.batch[lane];
+      if (pick == kSearchNewton)
+        search_trip<REBUILD, false>(b, sc, ctl, w, s, SHL_SMOOTH_EVAL_FGH);
+      else if (pick == kSearchTrial)
+        search_trip<REBUILD, false>(b, sc, ctl, w, s, SHL_SMOOTH_EVAL_TRIAL);
+      else
+        search_trip_deep<REBUILD>(b, sc, ctl, w, s);
+    }
+    __syncwarp();
   }
   if (lane == 0) {
     __threadfence();
@@ -1279,7 +1458,8 @@ static uint32_t search_grid() {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_smooth_search<REBUILD>, kSearchBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_smooth_search<REBUILD>, kSearchBlock,
+                                                  sizeof(SearchPool) * (kSearchBlock / 32));
     return (uint32_t)(sms > 0 ? sms : 152) * (uint32_t)(per_sm > 0 ? per_sm : 1);
   }();
   return g;
@@ -1288,21 +1468,27 @@ static uint32_t search_grid() {
 void launch_smooth_search(const DevBuf& b, const StepConst& sc, bool rebuild, cudaStream_t s) {
   uint32_t g = nblk(sc.F);
   if (g > 8 * 152) g = 8 * 152;
+  if (sc.F > sc.irr_first && g < 152) g = 152;  // the irregular children, hundreds per face
+  constexpr size_t smem = sizeof(SearchPool) * (kSearchBlock / 32);
   k_limit_coeffs<<<g, kBlock, 0, s>>>(b, sc, rebuild);
   if (rebuild)
-    k_smooth_search<true><<<search_grid<true>(), kSearchBlock, 0, s>>>(b, sc);
+    k_smooth_search<true><<<search_grid<true>(), kSearchBlock, smem, s>>>(b, sc);
   else
-    k_smooth_search<false><<<search_grid<false>(), kSearchBlock, 0, s>>>(b, sc);
+    k_smooth_search<false><<<search_grid<false>(), kSearchBlock, smem, s>>>(b, sc);
 }
 
-// k_csr_sort_big and k_rb_narrow take more than the default 48 KB of shared memory; called
-// once per device before its first launch
+// kernels that take more than the default 48 KB of shared memory; called once
+// per device before their first launch
 cudaError_t init_contact_kernels() {
-  const cudaError_t e = cudaFuncSetAttribute((const void*)k_rb_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(PairWork));
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute((const void*)k_csr_sort_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(kCsrSortBigCap * 4));
+  const auto set = [](const void* f, size_t bytes) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  cudaError_t e = set((const void*)k_rb_narrow, sizeof(PairWork));
+  if (e == cudaSuccess) e = set((const void*)k_csr_sort_big, kCsrSortBigCap * 4);
+  constexpr size_t pool = sizeof(SearchPool) * (kSearchBlock / 32);
+  if (e == cudaSuccess) e = set((const void*)k_smooth_search<true>, pool);
+  if (e == cudaSuccess) e = set((const void*)k_smooth_search<false>, pool);
+  return e;
 }
 
 void launch_contact_csr(const DevBuf& b, const StepConst& sc, cudaStream_t s) {

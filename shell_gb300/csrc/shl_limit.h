@@ -228,10 +228,60 @@ SHL_HD void shl_limit_poly(const double P[15][3], double v, double w, int order,
   }
 }
 
+/* The regular child of an irregular patch's n-th subdivision step that holds
+ * (v, w): level n and child k; (v, w) become the child's own coordinates and
+ * j1 is the derivative of the map. */
+SHL_HD void shl_limit_child(double* v, double* w, int* n_out, int* k_out, double* j1)
+{
+  const int n = shl_rescale_irregular(v, w);
+  *n_out = n;
+  if (*v > 0.5) {
+    *k_out = 0;
+    *v = SHL_SUB(SHL_MUL(2.0, *v), 1.0);
+    *w = SHL_MUL(2.0, *w);
+    *j1 = ldexp(1.0, n);
+  } else if (*w > 0.5) {
+    *k_out = 2;
+    *v = SHL_MUL(2.0, *v);
+    *w = SHL_SUB(SHL_MUL(2.0, *w), 1.0);
+    *j1 = ldexp(1.0, n);
+  } else {
+    *k_out = 1;
+    *v = SHL_SUB(1.0, SHL_MUL(2.0, *v));
+    *w = SHL_SUB(1.0, SHL_MUL(2.0, *w));
+    *j1 = -ldexp(1.0, n);
+  }
+}
+
+/* Component c of control point s of that child: a table row of the patch nodes
+ * (fused multiply-adds over the nonzero weights). */
+SHL_HD double shl_limit_child_point(const shl_limit_patch* pt, int n, int k, int s, int c)
+{
+  const int np = pt->N + 6;
+  const double* T = pt->tab + (size_t)((n - 1) * 3 + k) * 12 * (size_t)np;
+  double Q = 0.0;
+  for (int j = 0; j < np; ++j) {
+    const double t = T[s * np + j];
+    if (t == 0.0) continue;
+    Q = SHL_FMA(t, pt->base[3 * (size_t)pt->ids[(size_t)j * pt->stride] + c], Q);
+  }
+  return Q;
+}
+
+SHL_HD void shl_limit_coeffs_child(const shl_limit_patch* pt, int n, int k, double P[15][3])
+{
+  SHL_UNROLL
+  for (int m = 0; m < 15; ++m) P[m][0] = P[m][1] = P[m][2] = 0.0;
+  SHL_UNROLL
+  for (int s = 0; s < 12; ++s)
+    shl_limit_add_point(P, s, shl_limit_child_point(pt, n, k, s, 0), shl_limit_child_point(pt, n, k, s, 1),
+                        shl_limit_child_point(pt, n, k, s, 2));
+  shl_limit_scale(P);
+}
+
 /* Limit surface of a patch at (v, w) (outputs as shl_limit_poly).  An
  * irregular patch is evaluated in the regular child of the n-th subdivision
- * step that holds (v, w), whose control points are table rows of the patch
- * nodes (each formed by fused multiply-adds over the nonzero weights). */
+ * step that holds (v, w). */
 SHL_HD void shl_limit_eval(const shl_limit_patch* pt, double v, double w, int order, double out[6][3])
 {
   double P[15][3];
@@ -239,44 +289,11 @@ SHL_HD void shl_limit_eval(const shl_limit_patch* pt, double v, double w, int or
   if (pt->N == 6) {
     shl_limit_coeffs_regular(pt, P);
   } else {
-    const int n = shl_rescale_irregular(&v, &w);
-    int k;
-    if (v > 0.5) {
-      k = 0;
-      v = SHL_SUB(SHL_MUL(2.0, v), 1.0);
-      w = SHL_MUL(2.0, w);
-      j1 = ldexp(1.0, n);
-    } else if (w > 0.5) {
-      k = 2;
-      v = SHL_MUL(2.0, v);
-      w = SHL_SUB(SHL_MUL(2.0, w), 1.0);
-      j1 = ldexp(1.0, n);
-    } else {
-      k = 1;
-      v = SHL_SUB(1.0, SHL_MUL(2.0, v));
-      w = SHL_SUB(1.0, SHL_MUL(2.0, w));
-      j1 = -ldexp(1.0, n);
-    }
-    const int np = pt->N + 6;
-    const double* T = pt->tab + (size_t)((n - 1) * 3 + k) * 12 * (size_t)np;
-    for (int m = 0; m < 15; ++m) P[m][0] = P[m][1] = P[m][2] = 0.0;
-    SHL_UNROLL
-    for (int s = 0; s < 12; ++s) {
-      double Q0 = 0.0, Q1 = 0.0, Q2 = 0.0;
-      for (int j = 0; j < np; ++j) {
-        const double t = T[s * np + j];
-        if (t == 0.0) continue;
-        const double* x = pt->base + 3 * (size_t)pt->ids[(size_t)j * pt->stride];
-        Q0 = SHL_FMA(t, x[0], Q0);
-        Q1 = SHL_FMA(t, x[1], Q1);
-        Q2 = SHL_FMA(t, x[2], Q2);
-      }
-      shl_limit_add_point(P, s, Q0, Q1, Q2);
-    }
-    shl_limit_scale(P);
+    int n, k;
+    shl_limit_child(&v, &w, &n, &k, &j1);
+    shl_limit_coeffs_child(pt, n, k, P);
   }
   shl_limit_poly(P, v, w, order, j1, out);
 }
-
 
 #endif /* SHL_LIMIT_H_ */

@@ -230,6 +230,7 @@ SHL_HD int shl_smooth_direction(const double* g, double H[4][4], const unsigned*
     for (int b = 0; b < m; ++b) Hr[a][b] = SHL_MUL(SHL_MUL(S[a], Hr[a][b]), S[b]);
   }
   double mu = 0.0, L[4][4], y[4];
+  int bad = 0;
   for (int attempt = 0; attempt < 24; ++attempt) {
     bool ok = true;
     for (int a = 0; a < m && ok; ++a)
@@ -238,7 +239,7 @@ SHL_HD int shl_smooth_direction(const double* g, double H[4][4], const unsigned*
         if (a == b) s = SHL_ADD(s, mu);
         for (int k = 0; k < b; ++k) s = SHL_SUB(s, SHL_MUL(L[a][k], L[b][k]));
         if (a == b) {
-          if (!(s > 1e-14)) { ok = false; break; }
+          if (!(s > 1e-14)) { ok = false; bad = a; break; }
           L[a][a] = SHL_SQRT(s);
         } else {
           L[a][b] = SHL_DIV(s, L[b][b]);
@@ -263,7 +264,43 @@ SHL_HD int shl_smooth_direction(const double* g, double H[4][4], const unsigned*
       }
       return mu > 0.0 ? 1 : 0;
     }
-    mu = mu == 0.0 ? 1e-10 : SHL_MUL(mu, 10.0);
+    /* Two in five of a folded shell's steps need a shift, most of them of 1e-2
+     * to 1, and each smaller one is a factorisation that fails.  The first
+     * failure at pivot `bad` shows a direction of negative curvature,
+     * x = (-L_11^-T l, 1) with l the failed row: shifts that leave
+     * x^T (Hr + mu I) x clearly negative must fail too and are passed over: a
+     * factorisation that completes has a backward error below 1e-14 of the
+     * diagonal, and 1e-12 of all terms is allowed here (x need not be exact). */
+    if (attempt == 0) {
+      float x[4], xx = 0.0f;
+      for (int a = bad; a >= 0; --a) {
+        x[a] = 1.0f;
+        if (a < bad) {
+          float t = (float)L[bad][a];
+          for (int k = a + 1; k < bad; ++k) t += (float)L[k][a] * x[k];
+          x[a] = -t / (float)L[a][a];
+        }
+        xx += x[a] * x[a];
+      }
+      double q = 0.0, qa = 0.0;
+      for (int a = 0; a <= bad; ++a)
+        for (int b = 0; b <= a; ++b) {
+          const double t = ((double)(a == b ? x[a] : 2.0f * x[a]) * (double)x[b]) * Hr[a][b];
+          q += t;
+          qa += fabs(t);
+        }
+      /* xx, the threshold and the running m32 are within 1e-6 of the exact ones */
+      const float thr = (float)(-q - 1e-12 * qa);
+      float m32 = 1e-10f;
+      mu = 1e-10;
+      while (attempt < 22 && m32 * xx * 1.00001f + 2e-12f * (1.0f + xx) < thr) {
+        ++attempt;
+        m32 *= 10.0f;
+        mu = SHL_MUL(mu, 10.0);
+      }
+    } else {
+      mu = SHL_MUL(mu, 10.0);
+    }
   }
   /* not reached for finite input: scaled projected steepest descent */
   for (int a = 0; a < m; ++a) {
