@@ -317,8 +317,9 @@ shl_status shl_get_element_fields(shl_ctx* ctx, double* kGauss, double* kMean, d
  * basis contractions): shl_create times the shapes of the context's path on
  * its mesh and keeps the fastest (autotuning).  shl_set_element_variant forces
  * one (0-10 FP64, 11-13 FP32; 0 and 5 keep the displacement contraction in
- * FP64, 6-10 compute in double-float, 10 in one round of faces: one block of
- * 544 threads per SM, a face per thread) or, with -1, tunes again; shl_get_element_variant
+ * FP64, 6-10 compute in double-float: 6-8 with a face's components on three
+ * lanes, 9 and 10 with a face per thread, 10 in one round of faces) or, with -1,
+ * tunes again; shl_get_element_variant
  * returns the choice, its name and the tuning times of all
  * SHL_ELEMENT_VARIANTS (ms, 0 = not timed; tuned_ms holds that many floats).
  * No counterpart in the reference. */

@@ -61,6 +61,8 @@ struct shl_ctx {
   ElemGroups eg{};                 // 256-thread block ranges (the no-allocation path)
   ElemGroups eg_bs[3]{};           // block ranges for 64, 128, 256 threads per block
   uint32_t blocks_bs[3]{};
+  ElemGroups eg_split{};           // component-split kernels: block_start counts warps of ten faces
+  uint32_t split_warps = 0;
   int var64 = -1, var32 = kFirstFp32Variant;  // chosen element-kernel variants (-1: not set yet)
   float variant_ms[kNumElemVariants]{};      // tuning times (0: not timed)
   std::vector<void*> allocs;
@@ -110,6 +112,11 @@ ElemLaunch elem_launch(const shl_ctx* c, const StepConst& sc) {
     el.eg = c->eg_bs[0];
     return el;
   }
+  if (kElemVariants[el.variant].pairs == 2) {
+    el.blocks = c->split_warps;
+    el.eg = c->eg_split;
+    return el;
+  }
   const int k = bs_index(kElemVariants[el.variant].block);
   el.blocks = c->blocks_bs[k];
   el.eg = c->eg_bs[k];
@@ -148,6 +155,47 @@ shl_status upload(shl_ctx* c, T* dst, const T* src, size_t n) {
   return SHL_OK;
 }
 
+#define SHL_TRY(expr)             \
+  do {                            \
+    shl_status s_ = (expr);       \
+    if (s_ != SHL_OK) return s_;  \
+  } while (0)
+
+// The face constants by rows of float pairs (DevBuf::face_soa) from the split
+// records, for a face-per-thread variant forced on a context without them.
+void split_to_soa(const Setup& S, std::vector<float>& out) {
+  out.assign((size_t)2 * F32_COUNT * S.F, 0.f);
+  const int map[][2] = {{F32_JXW, SF_JXW}, {F32_L0, SF_L0}, {F32_K, SF_K}, {F32_D, SF_D}};
+  const int vec[][2] = {{F32_X0, SF_X}, {F32_A10, SF_A1}, {F32_A20, SF_A2}, {F32_D10, SF_D1}, {F32_D20, SF_D2},
+                        {F32_D30, SF_D3}, {F32_G0, SF_G}, {F32_N0, SF_N}, {F32_H00, SF_H}, {F32_H11, SF_H + 3}};
+  for (const PatchGroup& g : S.groups)
+    for (uint32_t i = g.first; i < g.first + g.count; ++i) {
+      const double* r = &S.split[(size_t)kSplitStride * i];
+      auto put = [&](int fld, double x) {
+        const float h = (float)x;
+        out[(size_t)fld * S.F + i] = h;
+        out[(size_t)(F32_COUNT + fld) * S.F + i] = (float)(x - (double)h);
+      };
+      for (int k = 0; k < 4; ++k) put(F32_R00 + k, r[SF_R00 + k] * (g.valence == 6 ? 324.0 : 1.0));
+      for (const auto& m : map) put(m[0], r[m[1]]);
+      for (const auto& v : vec)
+        for (int k = 0; k < 3; ++k) put(v[0] + k, r[v[1] + k]);
+    }
+}
+
+// the faces' split records as float pairs
+shl_status upload_split(shl_ctx* c) {
+  const std::vector<double>& r = c->S.split;
+  std::vector<float> t(2 * r.size());
+  for (size_t k = 0; k < r.size(); ++k) {
+    t[2 * k] = (float)r[k];
+    t[2 * k + 1] = (float)(r[k] - (double)t[2 * k]);
+  }
+  SHL_TRY(upload(c, c->b.face_df, t.data(), t.size()));
+  SHL_CUDA_TRY(cudaStreamSynchronize(c->stream));  // t is released here
+  return SHL_OK;
+}
+
 // the control block travels through a pinned host copy (one DMA, no staging)
 shl_status ctl_get(shl_ctx* c, Ctl& h) {
   Ctl* dst = c->h_ctl ? c->h_ctl : &h;
@@ -178,12 +226,6 @@ shl_status check_launch(const char* where) {
 }
 
 
-
-#define SHL_TRY(expr)             \
-  do {                            \
-    shl_status s_ = (expr);       \
-    if (s_ != SHL_OK) return s_;  \
-  } while (0)
 
 // Makes the corrector-side linked-cell pass that fused steps may have left
 // pending, so the candidate list and du_sum are those of the unfused sequence
@@ -502,21 +544,20 @@ namespace {
 // (c->S, one shell or a merged batch) is built; pscale: per original face.
 // The FP64 path's arithmetic: 0 = both basis contractions in FP64, 1 = the
 // displacement contraction as float pairs (24-26 % faster than 0 at levels 6
-// and 7), 2 = double-float throughout: the relative-displacement formulation
-// in float pairs on the FP32 pipe, shares kept as pairs and added in
-// double-float by the gather (element kernel 14 % faster than 1 at level 6,
-// 34 % at level 7; forces within 1e-14 of FP64).  Fixed for all contexts, so
-// that results do not depend on which launch shape a context picks (the
-// per-face arithmetic of a variant does not depend on its shape).
-constexpr int kFp64Pairs = 2;
+// and 7), 2 = the component-split kernel and 3 = a face per thread, both in
+// double-float on the FP32 pipe with the shares kept as pairs and added in
+// double-float by the gather.  Fixed by the contact mode, so that results do not
+// depend on which launch shape a context picks (the per-face arithmetic of a
+// variant does not depend on its shape).
+int fp64_arithmetic(const StepConst& sc) { return sc.smooth ? 3 : 2; }
 
 // step constants that follow the FP64 variant: its share format
-void apply_variant(shl_ctx* c) { c->sc.qe_df = kElemVariants[c->var64].pairs == 2 ? 1 : 0; }
+void apply_variant(shl_ctx* c) { c->sc.qe_df = kElemVariants[c->var64].pairs >= 2 ? 1 : 0; }
 
-// first FP64 variant of the fixed arithmetic (the FP64 launch of FP32 contexts)
-int default_var64() {
+// first FP64 variant of the context's arithmetic (the FP64 launch of FP32 contexts)
+int default_var64(const StepConst& sc) {
   for (int v = 0; v < kFirstFp32Variant; ++v)
-    if (kElemVariants[v].pairs == kFp64Pairs) return v;
+    if (kElemVariants[v].pairs == fp64_arithmetic(sc)) return v;
   return 0;
 }
 
@@ -533,7 +574,7 @@ shl_status tune_elements(shl_ctx* c) {
   int best_v = -1;
   for (int v = 0; v < kNumElemVariants; ++v) {
     const bool v32 = v >= kFirstFp32Variant;
-    if (v32 != fp32 || (!v32 && kElemVariants[v].pairs != kFp64Pairs)) continue;
+    if (v32 != fp32 || (!v32 && kElemVariants[v].pairs != fp64_arithmetic(c->sc))) continue;
     if (fp32) c->var32 = v; else c->var64 = v;
     const ElemLaunch el = elem_launch(c, c->sc);
     launch_elements(c->b, c->sc, el, c->stream);
@@ -600,8 +641,10 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
     ALLOC(b.up32, (size_t)V);
     ALLOC(b.face32, (size_t)F32_COUNT * F);
   } else {
-    ALLOC(b.face_df, (size_t)2 * F32_COUNT * F);
+    ALLOC(b.face_df, (size_t)2 * kSplitStride * F);
+    if (params->shell_shell_contact == SHL_CONTACT_SMOOTH) ALLOC(b.face_soa, S.face_soa.size());
   }
+  ALLOC(b.patch12, 12 * (size_t)S.groups[0].count);
   ALLOC(b.qe, fp32 ? 1 : 3 * (size_t)S.n_slots_total);
   ALLOC(b.gather_ptr, V + 1);
   ALLOC(b.slot_pos, S.slot_pos.size());
@@ -733,7 +776,12 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
   if ((st = upload(c, b.C, S.C.data(), nd)) != SHL_OK) return fail(st);
   if ((st = upload(c, b.face, S.face.data(), S.face.size())) != SHL_OK) return fail(st);
   if (fp32 && (st = upload(c, b.face32, S.face32.data(), S.face32.size())) != SHL_OK) return fail(st);
-  if (!fp32 && (st = upload(c, b.face_df, S.face_df.data(), S.face_df.size())) != SHL_OK) return fail(st);
+  if (!fp32 && (st = upload_split(c)) != SHL_OK) return fail(st);
+  if (b.face_soa && (st = upload(c, b.face_soa, S.face_soa.data(), S.face_soa.size())) != SHL_OK) return fail(st);
+  std::vector<int32_t> patch12(12 * (size_t)S.groups[0].count);
+  for (uint32_t i = 0; i < S.groups[0].count; ++i)
+    for (int k = 0; k < 12; ++k) patch12[12 * (size_t)i + k] = S.patch[(size_t)k * F + i];
+  if (!patch12.empty() && (st = upload(c, b.patch12, patch12.data(), patch12.size())) != SHL_OK) return fail(st);
   if ((st = upload(c, b.patch, S.patch.data(), S.patch.size())) != SHL_OK) return fail(st);
   if ((st = upload(c, b.gather_ptr, S.gather_ptr.data(), S.gather_ptr.size())) != SHL_OK) return fail(st);
   if ((st = upload(c, b.slot_pos, S.slot_pos.data(), S.slot_pos.size())) != SHL_OK) return fail(st);
@@ -792,17 +840,31 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
     double* d_basis = nullptr;
     if ((st = dev_alloc(c, &d_basis, basis.size())) != SHL_OK) return fail(st);
     if ((st = upload(c, d_basis, basis.data(), basis.size())) != SHL_OK) return fail(st);
+    std::vector<float2> pairs(basis.size());
+    for (size_t k = 0; k < basis.size(); ++k) {
+      pairs[k].x = (float)basis[k];
+      pairs[k].y = (float)(basis[k] - (double)pairs[k].x);
+    }
     std::vector<float> basis32(basis.begin(), basis.end());
     float* d_basis32 = nullptr;
     if ((st = dev_alloc(c, &d_basis32, basis32.size())) != SHL_OK) return fail(st);
     if ((st = upload(c, d_basis32, basis32.data(), basis32.size())) != SHL_OK) return fail(st);
+    float2* d_pairs = nullptr;
+    if ((st = dev_alloc(c, &d_pairs, pairs.size())) != SHL_OK) return fail(st);
+    if ((st = upload(c, d_pairs, pairs.data(), pairs.size())) != SHL_OK) return fail(st);
     c->eg.n = (int32_t)gd.size();
     for (size_t k = 0; k < gd.size(); ++k) c->eg.g[k] = gd[k];
     c->eg.basis = d_basis;
+    c->eg.basis_df = d_pairs;
     c->eg.basis32 = d_basis32;
     for (int k = 0; k < 3; ++k) {
       c->eg_bs[k] = c->eg;
       for (size_t q = 0; q < gd_bs[k].size(); ++q) c->eg_bs[k].g[q] = gd_bs[k][q];
+    }
+    c->eg_split = c->eg;
+    for (int q = 0; q < c->eg.n; ++q) {
+      c->eg_split.g[q].block_start = c->split_warps;
+      c->split_warps += (c->eg.g[q].count + kSplitFaces - 1) / kSplitFaces;
     }
   }
 
@@ -841,7 +903,7 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
   sc.smooth = smooth ? 1 : 0;
   sc.irr_first = irr_first;
   sc.irr_levels = irr_levels;
-  c->var64 = default_var64();
+  c->var64 = default_var64(sc);
   apply_variant(c);
   for (int k = 0; k < 13; ++k) sc.stab_off[k] = stab_off[k];
   sc.friction = (contact && (p.mu_s != 0 || p.mu_d != 0)) ? 1 : 0;
@@ -1759,8 +1821,12 @@ shl_status shl_residual(shl_ctx* c, double pressure, int flags, double* rel, dou
   }
   if (fp64 && ctx32 && !c->qe64) SHL_TRY(dev_alloc(c, &c->qe64, 3 * (size_t)c->S.n_slots_total));
   if (fp64 && ctx32 && !c->b.face_df) {  // the double-float FP64 path's constants
-    SHL_TRY(dev_alloc(c, &c->b.face_df, c->S.face_df.size()));
-    SHL_TRY(upload(c, c->b.face_df, c->S.face_df.data(), c->S.face_df.size()));
+    SHL_TRY(dev_alloc(c, &c->b.face_df, 2 * c->S.split.size()));
+    SHL_TRY(upload_split(c));
+    if (c->sc.smooth) {
+      SHL_TRY(dev_alloc(c, &c->b.face_soa, c->S.face_soa.size()));
+      SHL_TRY(upload(c, c->b.face_soa, c->S.face_soa.data(), c->S.face_soa.size()));
+    }
   }
   if (correct && !c->b.fcorr) {
     SHL_TRY(dev_alloc(c, &c->b.fcorr, nd));
@@ -2007,6 +2073,14 @@ shl_status shl_set_element_variant(shl_ctx* c, int variant) {
   if (variant >= kNumElemVariants || (variant >= kFirstFp32Variant) != (c->sc.fp32 != 0)) {
     g_err = "element variant does not exist for this precision";
     return SHL_ERR_ARG;
+  }
+  if (kElemVariants[variant].pairs == 3 && !c->b.face_soa) {
+    // the face-per-thread kernels read the constants row by row
+    std::vector<float> soa;
+    split_to_soa(c->S, soa);
+    SHL_TRY(dev_alloc(c, &c->b.face_soa, soa.size()));
+    SHL_TRY(upload(c, c->b.face_soa, soa.data(), soa.size()));
+    SHL_CUDA_TRY(cudaStreamSynchronize(c->stream));
   }
   if (c->sc.fp32) c->var32 = variant; else c->var64 = variant;
   apply_variant(c);

@@ -53,29 +53,32 @@ struct ElemGroups {
   GroupDesc g[kMaxGroups];
   int32_t n;
   const double* basis;
+  const float2* basis_df;  // the same as float pairs
   const float* basis32;
 };
 
 // An element-kernel variant: threads per block, arithmetic (0 FP64, 1 the
-// displacement contraction as float pairs, 2 double-float throughout;
-// FP32-path variants use 0) and a name for reports.
+// displacement contraction as float pairs, 2 component-split in double-float, 3
+// double-float with a face per thread; FP32-path variants use 0) and a name for
+// reports.
 struct ElemVariant {
   int block;
   int pairs;
   const char* name;
 };
 constexpr int kNumElemVariants = SHL_ELEMENT_VARIANTS;
-constexpr int kFirstFp32Variant = 11;
-// the one-round double-float element kernel (variant kFlatVariant): one block
-// of 544 threads (17 warps, 120 registers each) per SM, one face per thread
+constexpr int kSplitFaces = 10;  // faces per warp of the component-split kernel
+// the one-round double-float kernel: one block of 544 threads (17 warps, 120
+// registers each) per SM, one face per thread
 constexpr int kFlatVariant = 10;
 constexpr int kFlatBlock = 544;
+constexpr int kFirstFp32Variant = 11;
 extern const ElemVariant kElemVariants[kNumElemVariants];
 
 // The element launch of a context: variant, grid and patch-group block ranges for its block size.
 struct ElemLaunch {
   int variant;
-  uint32_t blocks;
+  uint32_t blocks;   // split variants: warps of ten faces
   ElemGroups eg;
 };
 
@@ -223,10 +226,12 @@ struct DevBuf {
   int32_t* patch;     // patch_rows * F, slot-major
   double* qe;         // 3 per element-force slot, in gather order (slot_pos)
   float* face32;      // F32_COUNT * F (FP32 element path)
-  float* face_df;     // 2 * F32_COUNT * F: the same constants as float pairs (double-float FP64 path)
+  float* face_df;     // kSplitStride float pairs per face (FP64 path: the component-split kernel)
+  float* face_soa;    // 2 * F32_COUNT * F: the FP32 constants as float pairs (SMOOTH contact: hi rows, then lo rows)
+  int32_t* patch12;   // regular faces: 12 patch node ids per face
   float* qe32;        // 3 per element-force slot, in gather order (FP32 element path)
   float4* up32;       // V, FP32 copy of u_pred (x, y, z, 0; FP32 element path)
-  float4* upk;        // 2V, u_pred as float pairs: [2n] = hi (x, y, z, 0), [2n + 1] = lo (the FP64 path's contractions)
+  float4* upk;        // 2V, u_pred as float pairs: [2n] = (hi x, lo x, hi y, lo y), [2n + 1] = (hi z, lo z, 0, 0)
   // element force shares are stored in gather order (node by node, ascending
   // element-force slot): slot_pos maps a (face, slot) to its place, and node n's
   // shares are qe[gather_ptr[n] .. gather_ptr[n + 1])

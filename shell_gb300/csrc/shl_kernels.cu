@@ -27,6 +27,7 @@
 #include "shl_internal.cuh"
 #include "shl_df.cuh"
 #include "shl_pairs.cuh"
+#include "shl_split.cuh"
 
 namespace shl {
 
@@ -497,8 +498,8 @@ __device__ __forceinline__ double predict_node(const DevBuf& b, const StepConst&
   if (sc.fp32) {
     b.up32[n] = make_float4(u32[0], u32[1], u32[2], 0.f);
   } else {
-    b.upk[2 * (size_t)n] = make_float4(uh[0], uh[1], uh[2], 0.f);
-    b.upk[2 * (size_t)n + 1] = make_float4(ul[0], ul[1], ul[2], 0.f);
+    b.upk[2 * (size_t)n] = make_float4(uh[0], ul[0], uh[1], ul[1]);
+    b.upk[2 * (size_t)n + 1] = make_float4(uh[2], ul[2], 0.f, 0.f);
   }
   return __dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2]));
 }
@@ -714,8 +715,8 @@ __device__ __forceinline__ void set_positions(const DevBuf& b, const StepConst& 
     df_split(up[c], uh[c], ul[c]);
   }
   if (sc.fp32) b.up32[n] = make_float4((float)up[0], (float)up[1], (float)up[2], 0.f);
-  b.upk[2 * (size_t)n] = make_float4(uh[0], uh[1], uh[2], 0.f);
-  b.upk[2 * (size_t)n + 1] = make_float4(ul[0], ul[1], ul[2], 0.f);
+  b.upk[2 * (size_t)n] = make_float4(uh[0], ul[0], uh[1], ul[1]);
+  b.upk[2 * (size_t)n + 1] = make_float4(uh[2], ul[2], 0.f, 0.f);
 }
 
 // The state from (hu, hv, ha) or to them: host memory that the device reads and
@@ -789,8 +790,8 @@ __device__ __forceinline__ ElemOut element_force(uint32_t i, int np_rt, uint32_t
     for (int s = 0; s < (NP > 0 ? NP : kMaxSlots); ++s) {
       if (NP == 0 && s >= np) break;
       const int nd = __ldg(&b.patch[(size_t)s * F + i]);
-      const float4 h4 = __ldg(&b.upk[2 * (size_t)nd]), l4 = __ldg(&b.upk[2 * (size_t)nd + 1]);
-      const float uh[3] = {h4.x, h4.y, h4.z}, ul[3] = {l4.x, l4.y, l4.z};
+      const float4 xy = __ldg(&b.upk[2 * (size_t)nd]), z0 = __ldg(&b.upk[2 * (size_t)nd + 1]);
+      const float uh[3] = {xy.x, xy.z, z0.x}, ul[3] = {xy.y, xy.w, z0.y};
 #pragma unroll
       for (int k = 0; k < 6; ++k) {
         const float wh = Bh[6 * s + k], wl = Bl[6 * s + k];
@@ -1153,11 +1154,17 @@ __device__ __forceinline__ ElemOut element_force32(uint32_t i, int np_rt, uint32
 
 // Element kernels are compiled in several launch shapes (threads per block,
 // blocks per SM, hence registers per thread) -- and for the FP64 path with the
-// two basis contractions in FP64 or as float pairs; set-up times them on the
-// context's own mesh and keeps the fastest (shl_api.cu, tune_elements).  The
-// per-face arithmetic of one path does not depend on the launch shape.  The
-// totals of the per-face measurements are summed by k_elem_totals.
-// FP64-class element force in double-float arithmetic on the FP32 pipe: the
+// displacement contraction in FP64 or as float pairs, and component-split in
+// double-float (shl_split.cuh); set-up times the shapes of the context's
+// arithmetic on its own mesh and keeps the fastest (shl_api.cu, tune_elements).
+// The per-face arithmetic does not depend on the launch shape.  The totals of
+// the per-face measurements are summed by k_elem_totals.
+// FP64-class element force in double-float arithmetic, one face per thread: the
+// arithmetic of contexts with SMOOTH contact, whose closest-point searches stop
+// within their tolerance wherever the last bits of the positions send them -- a
+// stored run or list goes on as it was started.  (Element forces are 1 % of such
+// a step; the component-split kernel of the other contexts rounds differently.)
+// The
 // relative-displacement formulation of element_force32 with every quantity a
 // float pair (about 48 significant bits), the constants from face_df (the
 // same balanced-frame values as face32, kept to 48 bits), the displacement
@@ -1198,7 +1205,7 @@ __device__ __forceinline__ ElemOut element_force_df(uint32_t i, int np_rt, uint3
     // slots in a rolled loop: the unrolled double-float code would not fit the instruction cache
 #pragma unroll 1
     for (int s = 0; s < np; ++s) {
-      float4 h4, l4;
+      float4 h4, l4;  // (hi x, lo x, hi y, lo y), (hi z, lo z, 0, 0)
       if (NP > 0) {
         h4 = su[(2 * s) * bs + t];
         l4 = su[(2 * s + 1) * bs + t];
@@ -1207,7 +1214,7 @@ __device__ __forceinline__ ElemOut element_force_df(uint32_t i, int np_rt, uint3
         h4 = __ldg(&b.upk[2 * (size_t)nd]);
         l4 = __ldg(&b.upk[2 * (size_t)nd + 1]);
       }
-      const float uh[3] = {h4.x, h4.y, h4.z}, ul[3] = {l4.x, l4.y, l4.z};
+      const float uh[3] = {h4.x, h4.z, l4.x}, ul[3] = {h4.y, h4.w, l4.y};
 #pragma unroll
       for (int k = 0; k < 6; ++k) {
         const float wh = Bh[6 * s + k], wl = Bl[6 * s + k];
@@ -1220,7 +1227,7 @@ __device__ __forceinline__ ElemOut element_force_df(uint32_t i, int np_rt, uint3
 #pragma unroll
       for (int c = 0; c < 3; ++c) df_quick_two_sum(gh[k][c], gl[k][c], G[k][c].h, G[k][c].l);
   }
-  const float* fd = b.face_df;
+  const float* fd = b.face_soa;
   // constant row r (hi rows 0..37, lo rows 38..75) in component r % 4 of this
   // thread's float4 entry r / 4 -- the entries that held its displacements
   static_assert(2 * F32_COUNT <= 4 * 2 * kDfStageSlots, "face constants exceed the staging column");
@@ -2331,33 +2338,34 @@ void launch_ctl_begin(Ctl* ctl, uint32_t n, uint32_t flags, cudaStream_t s) { k_
 const ElemVariant kElemVariants[kNumElemVariants] = {
     {256, 0, "fp64 256x1"},        {256, 1, "fp64 256x1 pair-G"}, {128, 1, "fp64 128x3 pair-G"},
     {64, 1, "fp64 64x5 pair-G"},   {64, 1, "fp64 64x6 pair-G"},   {64, 0, "fp64 64x5"},
-    {256, 2, "fp64 256x1 df"},     {128, 2, "fp64 128x3 df"},     {64, 2, "fp64 64x6 df"},
-    {64, 2, "fp64 64x8 df"},       {kFlatBlock, 2, "fp64 544x1 df flat"},
+    {128, 2, "fp64 128x5 split"},  {64, 2, "fp64 64x8 split"},    {64, 2, "fp64 64x12 split"},
+    {128, 3, "fp64 128x3 df"},     {kFlatBlock, 3, "fp64 544x1 df flat"},
     {256, 0, "fp32 256x2"},        {128, 0, "fp32 128x4"},        {64, 0, "fp32 64x8"}};
 
-// the double-float kernels take more than the default 48 KB of shared memory
-// (staging plus the basis table); called once per device before their first launch
+template <int BS, int MINB>
+static void launch_split(const DevBuf& b, const StepConst& sc, const ElemLaunch& el, cudaStream_t s) {
+  constexpr int warps = BS / 32;
+  k_elements_split<BS, MINB><<<(el.blocks + warps - 1) / warps, BS, warps * sizeof(SplitWarp), s>>>(b, sc, el.eg, el.blocks);
+}
+
+// attributes of the kernels with much shared memory; called once per device
+// before their first launch
 cudaError_t init_element_kernels() {
-  cudaError_t e = cudaSuccess;
-  auto set = [&](const void* f, int block) {
-    if (e != cudaSuccess) return;
-    e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)df_stage_bytes(block));
+  cudaError_t e = cudaFuncSetAttribute((const void*)k_contact_force<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(PairWork));
+  auto carveout = [&](const void* f) {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   };
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void*)k_contact_force<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(PairWork));
-  set((const void*)k_elements_df<256, 1>, 256);
-  set((const void*)k_elements_df<128, 3>, 128);
-  set((const void*)k_elements_df<64, 6>, 64);
-  set((const void*)k_elements_df<64, 8>, 64);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void*)k_elements_df_flat<kFlatBlock>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)flat_smem_bytes());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void*)k_elements_df_flat<kFlatBlock>,
-                             cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  carveout((const void*)k_elements_split<128, 5>);
+  carveout((const void*)k_elements_split<64, 8>);
+  carveout((const void*)k_elements_split<64, 12>);
+  auto set = [&](const void* f, size_t bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    carveout(f);
+  };
+  set((const void*)k_elements_df<128, 3>, df_stage_bytes(128));
+  set((const void*)k_elements_df_flat<kFlatBlock>, flat_smem_bytes());
   return e;
 }
 
@@ -2371,10 +2379,10 @@ void launch_elements(const DevBuf& b, const StepConst& sc, const ElemLaunch& el,
     case 3: k_elements<64, 5, true, false><<<nb, 64, 0, s>>>(b, sc, eg); break;
     case 4: k_elements<64, 6, true, false><<<nb, 64, 0, s>>>(b, sc, eg); break;
     case 5: k_elements<64, 5, false, false><<<nb, 64, 0, s>>>(b, sc, eg); break;
-    case 6: k_elements_df<256, 1><<<nb, 256, df_stage_bytes(256), s>>>(b, sc, eg); break;
-    case 7: k_elements_df<128, 3><<<nb, 128, df_stage_bytes(128), s>>>(b, sc, eg); break;
-    case 8: k_elements_df<64, 6><<<nb, 64, df_stage_bytes(64), s>>>(b, sc, eg); break;
-    case 9: k_elements_df<64, 8><<<nb, 64, df_stage_bytes(64), s>>>(b, sc, eg); break;
+    case 6: launch_split<128, 5>(b, sc, el, s); break;
+    case 7: launch_split<64, 8>(b, sc, el, s); break;
+    case 8: launch_split<64, 12>(b, sc, el, s); break;
+    case 9: k_elements_df<128, 3><<<nb, 128, df_stage_bytes(128), s>>>(b, sc, eg); break;
     case 10: k_elements_df_flat<kFlatBlock><<<nb, kFlatBlock, flat_smem_bytes(), s>>>(b, sc, eg); break;
     case 11: k_elements32<256, 2><<<nb, 256, 0, s>>>(b, sc, eg); break;
     case 12: k_elements32<128, 4><<<nb, 128, 0, s>>>(b, sc, eg); break;

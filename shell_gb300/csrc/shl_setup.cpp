@@ -347,7 +347,7 @@ bool build_setup(const shl_mesh& mesh, const shl_params& prm, Setup& S, std::str
 
   S.patch.assign((size_t)S.patch_rows * F, -1);
   S.face.assign((size_t)FF_COUNT * F, 0.0);
-  std::vector<double> face_bal((size_t)FF_COUNT * F, 0.0);  // balanced-frame constants (FP32 path)
+  std::vector<double> face_bal((size_t)FF_COUNT * F, 0.0);  // balanced-frame constants (FP32 and split records)
   S.Minv.assign(3 * (size_t)V, 0.0);
   S.C.assign(3 * (size_t)V, 0.0);
   auto Xn = [&](uint32_t n) { return V3{S.X[3 * n], S.X[3 * n + 1], S.X[3 * n + 2]}; };
@@ -482,14 +482,16 @@ bool build_setup(const shl_mesh& mesh, const shl_params& prm, Setup& S, std::str
   }
   // FP32 constants of the relative-displacement element path
   S.face32.assign((size_t)F32_COUNT * F, 0.0f);
-  S.face_df.assign((size_t)2 * F32_COUNT * F, 0.0f);
+  const bool soa = prm.shell_shell_contact == SHL_CONTACT_SMOOTH;
+  if (soa) S.face_soa.assign((size_t)2 * F32_COUNT * F, 0.0f);
   for (uint32_t i = 0; i < F; ++i) {
     auto get = [&](int fld) { return face_bal[(size_t)fld * F + i]; };
     auto put32 = [&](int fld, double x) {
       const float h = (float)x;
       S.face32[(size_t)fld * F + i] = h;
-      S.face_df[(size_t)fld * F + i] = h;
-      S.face_df[(size_t)(F32_COUNT + fld) * F + i] = (float)(x - (double)h);
+      if (!soa) return;
+      S.face_soa[(size_t)fld * F + i] = h;
+      S.face_soa[(size_t)(F32_COUNT + fld) * F + i] = (float)(x - (double)h);
     };
     const int map64[][2] = {{F32_R00, FF_R00}, {F32_R01, FF_R01}, {F32_R10, FF_R10}, {F32_R11, FF_R11},
                             {F32_JXW, FF_JXW}, {F32_X0, FF_X0}, {F32_X1, FF_X1}, {F32_X2, FF_X2},
@@ -509,6 +511,33 @@ bool build_setup(const shl_mesh& mesh, const shl_params& prm, Setup& S, std::str
     put32(F32_N2, n.z / L);
     put32(F32_L0, L);
   }
+
+  // records of the component-split element kernel
+  S.split.assign((size_t)kSplitStride * F, 0.0);
+  for (const PatchGroup& g : S.groups)
+    for (uint32_t i = g.first; i < g.first + g.count; ++i) {
+      auto get = [&](int fld) { return face_bal[(size_t)fld * F + i]; };
+      double* r = &S.split[(size_t)kSplitStride * i];
+      const double q1 = g.valence == 6 ? 324.0 : 1.0, q2 = g.valence == 6 ? 108.0 : 1.0;
+      const double R00 = get(FF_R00), R01 = get(FF_R01), R10 = get(FF_R10), R11 = get(FF_R11);
+      r[SF_R00] = R00 / q1; r[SF_R01] = R01 / q1; r[SF_R10] = R10 / q1; r[SF_R11] = R11 / q1;
+      r[SF_C11A] = R00 * R00 / q2; r[SF_C11B] = R10 * R10 / q2; r[SF_C11C] = 2 * R00 * R10 / q2;
+      r[SF_C22A] = R01 * R01 / q2; r[SF_C22B] = R11 * R11 / q2; r[SF_C22C] = 2 * R01 * R11 / q2;
+      r[SF_C12A] = R00 * R01 / q2; r[SF_C12B] = R10 * R11 / q2; r[SF_C12C] = (R01 * R10 + R00 * R11) / q2;
+      r[SF_JXW] = get(FF_JXW);
+      const int vec[][2] = {{SF_X, FF_X0}, {SF_A1, FF_A10}, {SF_A2, FF_A20}, {SF_D1, FF_D10}, {SF_D2, FF_D20},
+                            {SF_D3, FF_D30}, {SF_G, FF_G0}, {SF_B, FF_B0}};
+      for (const auto& v : vec)
+        for (int c = 0; c < 3; ++c) r[v[0] + c] = get(v[1] + c);
+      for (int k = 0; k < 6; ++k) r[SF_H + k] = get(FF_H00 + k);
+      r[SF_K] = get(FF_K);
+      r[SF_D] = get(FF_D);
+      const V3 a1{get(FF_A10), get(FF_A11), get(FF_A12)}, a2{get(FF_A20), get(FF_A21), get(FF_A22)};
+      const V3 n = cross(a1, a2);
+      const double L = norm(n);
+      r[SF_N] = n.x / L; r[SF_N + 1] = n.y / L; r[SF_N + 2] = n.z / L;
+      r[SF_L0] = L;
+    }
 
   for (double& c : S.C) c += prm.damping_gamma;
   for (double& m : S.Minv) {
@@ -644,7 +673,9 @@ bool merge_setups(std::vector<Setup>& shells, Setup& M, std::vector<uint32_t>& n
   M.patch.assign((size_t)M.patch_rows * F, -1);
   M.face.assign((size_t)FF_COUNT * F, 0.0);
   M.face32.assign((size_t)F32_COUNT * F, 0.0f);
-  M.face_df.assign((size_t)2 * F32_COUNT * F, 0.0f);
+  const bool soa = !shells[0].face_soa.empty();
+  if (soa) M.face_soa.assign((size_t)2 * F32_COUNT * F, 0.0f);
+  M.split.assign((size_t)kSplitStride * F, 0.0);
   for (uint32_t i = 0; i < F; ++i) {
     const uint32_t k = src[i].first, si = src[i].second;
     const Setup& S = shells[k];
@@ -654,7 +685,10 @@ bool merge_setups(std::vector<Setup>& shells, Setup& M, std::vector<uint32_t>& n
     }
     for (int fld = 0; fld < FF_COUNT; ++fld) M.face[(size_t)fld * F + i] = S.face[(size_t)fld * S.F + si];
     for (int fld = 0; fld < F32_COUNT; ++fld) M.face32[(size_t)fld * F + i] = S.face32[(size_t)fld * S.F + si];
-    for (int fld = 0; fld < 2 * F32_COUNT; ++fld) M.face_df[(size_t)fld * F + i] = S.face_df[(size_t)fld * S.F + si];
+    if (soa)
+      for (int fld = 0; fld < 2 * F32_COUNT; ++fld)
+        M.face_soa[(size_t)fld * F + i] = S.face_soa[(size_t)fld * S.F + si];
+    std::copy_n(&S.split[(size_t)kSplitStride * si], kSplitStride, &M.split[(size_t)kSplitStride * i]);
   }
   build_node_lists(M);
   // topological exclusion sets (self-contact), face ids offset shell by shell

@@ -55,6 +55,30 @@ enum FaceField32 {
   F32_COUNT
 };
 
+// Per-face constants of the component-split element kernel (one record of
+// kSplitStride values per face, internal order): the balanced material frame
+// (|k| = |j| = sqrt |b1 x b2|; reinit_mod's scaling degenerates on some faces).
+// On a regular patch R and the second-derivative coefficients C are divided by
+// the denominators of the basis derivatives (324 and 108).
+enum SplitField {
+  SF_R00, SF_R01, SF_R10, SF_R11,  // rotation onto the material frame
+  SF_C11A, SF_C11B, SF_C11C,       // R00^2, R10^2, 2 R00 R10
+  SF_C22A, SF_C22B, SF_C22C,       // R01^2, R11^2, 2 R01 R11
+  SF_C12A, SF_C12B, SF_C12C,       // R00 R01, R10 R11, R01 R10 + R00 R11
+  SF_JXW,
+  SF_X,                            // quadrature point, reference
+  SF_A1 = SF_X + 3, SF_A2 = SF_A1 + 3, SF_D1 = SF_A2 + 3, SF_D2 = SF_D1 + 3, SF_D3 = SF_D2 + 3,
+  SF_G = SF_D3 + 3,                // a_ref.ff1
+  SF_N = SF_G + 3,                 // unit normal and |a1 x a2| of the reference
+  SF_L0 = SF_N + 3,
+  SF_B,                            // a_ref.ff2
+  SF_H = SF_B + 3,                 // H00, H01, H02, H11, H12, H22
+  SF_K = SF_H + 6, SF_D,
+  SF_COUNT
+};
+constexpr int kSplitStride = 52;   // values per record: a multiple of 16 bytes as float pairs
+static_assert(SF_COUNT <= kSplitStride, "record size");
+
 struct PatchGroup {
   int valence;        // valence of the first vertex (6 = regular)
   int n_slots;        // valence + 6
@@ -77,7 +101,8 @@ struct Setup {
   std::vector<int32_t> patch;      // [slot * F + internal face], -1 for unused slots
   std::vector<double> face;        // [field * F + internal face]
   std::vector<float> face32;       // [FaceField32 * F + internal face]
-  std::vector<float> face_df;      // the same constants as float pairs: hi [fld * F + i], lo [(F32_COUNT + fld) * F + i]
+  std::vector<float> face_soa;     // SMOOTH contact: the same as float pairs, hi [fld * F + i], lo [(F32_COUNT + fld) * F + i]
+  std::vector<double> split;       // [internal face * kSplitStride + SplitField]
   std::vector<double> Minv, C;     // 3V node-major
   std::vector<uint32_t> gather_ptr;  // V+1
   std::vector<uint32_t> gather_ent;  // element-force slot (PatchGroup::slot_base), ascending per node
