@@ -132,9 +132,10 @@ struct Ctl {
   uint32_t paused;          // 1: steps_target reached, 2: stopping criterion true
   // cavity contact (ShellSystem.C:1600-1723)
   double cav_R[3];          // semi-axes of the current step
+  double cav_Rm[3];         // pipelined steps: semi-axes of the step being measured
   double Ecav, cavity_force;
   uint32_t Nc_cav;
-  uint32_t pad_cav;
+  uint32_t measure;         // pipelined steps: the corrector ended a step that is to be measured
   double sum_pcav, sum_Nc_cav, sum_Ecav;
   // dt-weighted sums (MovingAverage inputs)
   double sum_dt, sum_area, sum_volume, sum_Nc, sum_Ekin, sum_Etens, sum_Ebend, sum_Eself, sum_Efric,
@@ -240,7 +241,9 @@ struct DevBuf {
   uint32_t* tri;      // 3F original order
   uint32_t *perm;     // internal -> original
   double *area, *kG, *kM, *etens, *ebend;  // original order
+  double *area_odd, *kG_odd, *kM_odd, *etens_odd, *ebend_odd;  // the same fields of every other pipelined step
   double* partial;    // per-block partial sums
+  double* partial_v;  // those of the measurement (k_volume_end), which runs beside other kernels
   uint32_t *close_ptr, *close_list;
   // contact: per-face AABB (original order), size, cell ranges
   double *bmin, *bmax, *fsize;
@@ -348,10 +351,15 @@ void launch_elements(const DevBuf& b, const StepConst& sc, const ElemLaunch& el,
 void launch_contact_force(const DevBuf& b, const StepConst& sc, int cur, cudaStream_t s);
 // mode 2: adaptive attempt; mode 3: corrector fused with the next step's prediction
 // (reads the step's predicted positions from b.pn and writes the next ones there);
-// otherwise correct ? corrector : evaluation
+// mode 4: the same, and the end of the step and the scalar start of the next one;
+// mode 5: the last such step of a run (no start of a next one); otherwise
+// correct ? corrector : evaluation
 void launch_gather_correct(const DevBuf& b, const StepConst& sc, int mode, bool correct, double* f_out,
                            double* a_out, cudaStream_t s, RebuildCond rc = {0, 0});
-void launch_volume_end_step(const DevBuf& b, const StepConst& sc, bool end_step, cudaStream_t s);
+// the measurement totals and the volume (kVolTotals), with the end of the step
+// (kVolEndStep), or with the report's sums of a pipelined step (kVolMeasure)
+enum : int { kVolTotals = 0, kVolEndStep = 1, kVolMeasure = 2 };
+void launch_volume_end_step(const DevBuf& b, const StepConst& sc, int mode, cudaStream_t s);
 void launch_positions(const DevBuf& b, const StepConst& sc, cudaStream_t s);
 // u, v, a between the context and mapped page-locked host memory (device pointers of it)
 void launch_state_host(const DevBuf& b, const StepConst& sc, double* hu, double* hv, double* ha, bool load,

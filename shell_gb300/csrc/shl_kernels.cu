@@ -753,6 +753,51 @@ __global__ void k_positions(DevBuf b, StepConst sc) {
   set_positions(b, sc, n, up);
 }
 
+// The end of a step (one thread): its problem becomes the run's, the run halts or
+// pauses (ShellSystem.C:2901-2953, shell.C:314-318)
+__device__ void end_step_scalar(Ctl* ctl, const StepConst& sc) {
+  const int pr = ctl->problem;
+  if (pr > ctl->worst_problem) ctl->worst_problem = pr;
+  if (pr > 0 && ctl->first_problem_step == 0) ctl->first_problem_step = ctl->time_step;
+  ctl->steps_done += 1;
+  if (pr >= SHL_STOP_SIM || (sc.stop_on_problem && pr > 0) || ctl->error) ctl->halted = 1;
+  ctl->problem = 0;
+  // the next step's dt, after the measurement used this one (ShellSystem.C:1096-1098)
+  if (sc.adapt_every) set_newmark(ctl, sc, ctl->new_dt);
+  if (ctl->steps_done >= ctl->steps_target) ctl->paused |= 1u;
+  // stopping criterion, tested before the next step
+  if (sc.sfun_len > 0 && eval_program(sc.sfun, sc.sfun_len, ctl->time, 0.0) != 0.0) ctl->paused |= 2u;
+}
+
+// A pipelined corrector's scalars (one thread; a batch: all threads of the
+// block): the step ends here, its measurement being left to k_volume_end beside
+// the next step, and the next step starts unless the run stopped or this is the
+// run's last one (next = 0).
+__device__ void end_and_begin(const DevBuf& b, const StepConst& sc, const RebuildCond& rc, bool next) {
+  Ctl* ctl = b.ctl;
+  if (threadIdx.x == 0) {
+    ctl->measure = 1u;
+    for (int c = 0; c < 3; ++c) ctl->cav_Rm[c] = ctl->cav_R[c];
+    end_step_scalar(ctl, sc);
+  }
+  if (!next) return;
+  if (sc.n_cs) {
+    __syncthreads();
+    if (inactive(ctl)) {
+      if (threadIdx.x == 0) set_rebuild_cond(rc, ctl);
+      return;
+    }
+    if (threadIdx.x == 0) begin_step_scalar(ctl, sc, sc.dt);
+    __syncthreads();
+    batch_begin_check(b, sc, rc, true, false);
+    return;
+  }
+  if (inactive(ctl))
+    set_rebuild_cond(rc, ctl);
+  else
+    begin_step(ctl, sc, sc.dt, ctl->du2_pred, rc, true);
+}
+
 // ------------------------------------------------------------- elements --
 struct ElemOut {
   double etens, ebend, kg, km, area;
@@ -1734,10 +1779,14 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
   // mode 0: eval (write f_out / a_out), mode 1: step corrector, mode 2: adaptive
   // attempt, mode 3: step corrector fused with the next step's prediction (fixed
   // dt): the step's predicted positions are read from b.pn and the next ones
-  // written there, the corrected positions go to b.p
+  // written there, the corrected positions go to b.p; mode 4 and 5: pipelined
+  // steps, whose corrector also ends the step (and, in mode 4, starts the next)
   Ctl* ctl = b.ctl;
   if (inactive(ctl)) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) set_rebuild_cond(rc, ctl);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (mode >= 4) ctl->measure = 0u;
+      set_rebuild_cond(rc, ctl);
+    }
     return;
   }
   __shared__ double sh[kBlock / 32];
@@ -1748,7 +1797,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
     double f[3] = {0.0, 0.0, 0.0};
     // the node's state, loaded ahead of (and independently of) the share sums
     const size_t k3n = 3 * (size_t)n;
-    const bool corr = mode == 1 || mode == 3;
+    const bool corr = mode == 1 || mode >= 3;
     double s_vp[3], s_minv[3], s_c[3], s_up[3], s_u[3], s_x[3], s_m[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -1818,7 +1867,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
       // interaction with the cavity (ShellSystem.C:1600-1723)
       const CavityGeom cg = cavity_geom(ctl->cav_R, sc);
       const size_t k3 = 3 * (size_t)n;
-      const double* pp = mode == 3 ? b.pn : b.p;
+      const double* pp = mode >= 3 ? b.pn : b.p;
       const double p[3] = {pp[k3], pp[k3 + 1], pp[k3 + 2]};
       const double xr = (p[0] / cg.R_eff[0]) * (p[0] / cg.R_eff[0]);
       const double yr = (p[1] / cg.R_eff[1]) * (p[1] / cg.R_eff[1]);
@@ -1941,13 +1990,13 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
         an[c] = ap;
       }
     }
-    if (mode == 1 || mode == 3) du2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    if (mode == 3) du2_next = predict_node(b, sc, n, un, vnn, an, sc.dt, sc.nm8, sc.nm6, b.pn);
+    if (mode == 1 || mode >= 3) du2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    if (mode >= 3) du2_next = predict_node(b, sc, n, un, vnn, an, sc.dt, sc.nm8, sc.nm6, b.pn);
   }
   if (mode == 0) return;
-  if (sc.n_cs && (mode == 1 || mode == 3)) {
+  if (sc.n_cs && (mode == 1 || mode >= 3)) {
     shell_max_acc(b, sc, n, du2, 0);
-    if (mode == 3) shell_max_acc(b, sc, n, du2_next, 1);
+    if (mode >= 3) shell_max_acc(b, sc, n, du2_next, 1);
   }
   if (sc.cavity_contact) {
     const double r0 = block_sum(c_nc, sh), r1 = block_sum(c_e, sh), r2 = block_sum(c_ef, sh),
@@ -2007,7 +2056,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
   }
   const double m = block_max(du2, sh);
   const double ek = block_sum(0.5 * ekin, sh);
-  const double mn = mode == 3 ? block_max(du2_next, sh) : 0.0;
+  const double mn = mode >= 3 ? block_max(du2_next, sh) : 0.0;
   if (threadIdx.x == 0) {
     b.partial[(size_t)blockIdx.x * 8] = m;
     b.partial[(size_t)blockIdx.x * 8 + 1] = ek;
@@ -2021,19 +2070,20 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
     mmn = fmax(mmn, __ldcg(&b.partial[(size_t)k * 8 + 6]));
   }
   mm = block_max(mm, sh);
-  if (mode == 3) mmn = block_max(mmn, sh);
+  if (mode >= 3) mmn = block_max(mmn, sh);
   const double ekt = sum_partials(b.partial, 1, gridDim.x, sh);
   if (sc.n_cs) {  // a batch: each shell's own check_increment(true)
     if (threadIdx.x == 0) {
       ctl->Ekin = ekt;
       if (!isfinite(ekt)) register_problem(ctl, SHL_NOT_FINITE);
     }
-    batch_correct_check(b, sc, rc, mode == 3);
+    batch_correct_check(b, sc, rc, mode >= 3);
+    if (mode >= 4) end_and_begin(b, sc, rc, mode == 4);
     return;
   }
   if (threadIdx.x != 0) return;
   ctl->Ekin = ekt;
-  if (mode == 3) ctl->du2_pred = mmn;  // check_increment(false) of the next step, in k_begin_step
+  if (mode >= 3) ctl->du2_pred = mmn;  // check_increment(false) of the next step, in k_begin_step
   // check_increment(true)
   const double du_max = sqrt(mm);
   if (isfinite(du_max)) {
@@ -2047,8 +2097,9 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
   }
   if (!isfinite(ekt)) register_problem(ctl, SHL_NOT_FINITE);
   const uint32_t flag = (sc.contact && ctl->du_sum >= rebuild_tolerance(sc, ctl)) ? 1u : 0u;
-  if (mode == 3) {
+  if (mode >= 3) {
     ctl->rebuild_pending = flag;  // made by the next step's IF node, before its own pass
+    if (mode >= 4) end_and_begin(b, sc, rc, mode == 4);
     return;
   }
   ctl->rebuild = flag;
@@ -2119,9 +2170,11 @@ __global__ void __launch_bounds__(kBlock) k_correct_adapt(DevBuf b, StepConst sc
 }
 
 // ------------------------------------------------------ volume, end step --
-__global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, int end_step) {
+__global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, int mode) {
   Ctl* ctl = b.ctl;
-  if (inactive(ctl)) return;
+  const bool end_step = mode == kVolEndStep;
+  // a pipelined step was ended by its corrector, which may have stopped the run
+  if (mode == kVolMeasure ? ctl->measure == 0 : inactive(ctl)) return;
   if (end_step && sc.adapt_every && !ctl->accept) {
     // a repeated attempt ends no step; only a step size below the machine
     // precision (SHL_SMALL_TIMESTEP) ends the run (ShellSystem.C:1110-1117)
@@ -2151,16 +2204,16 @@ __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, i
   }
   block_sum_t<6>(v, sh);
   if (threadIdx.x == 0) {
-    double* pp = b.partial + (size_t)blockIdx.x * 8;
+    double* pp = b.partial_v + (size_t)blockIdx.x * 8;
     for (int k = 0; k < 6; ++k) pp[k] = v[k];
   }
   if (!last_block(&ctl->cnt[4])) return;
   double t[6];
-  sum_partials_t<6>(b.partial, gridDim.x, sh, t);
+  sum_partials_t<6>(b.partial_v, gridDim.x, sh, t);
   if (threadIdx.x != 0) return;
   ctl->Etens = t[0]; ctl->Ebend = t[1]; ctl->kGauss = t[2]; ctl->kMean = t[3]; ctl->area = t[4];
   ctl->volume = fabs(t[5] / 6.0) - ctl->area * 0.5 * sc.thickness;
-  if (!end_step) return;
+  if (mode == kVolTotals) return;
   const double dt = sc.adapt_every ? ctl->dt_cur : sc.dt;
   ctl->sum_dt += dt;
   ctl->sum_area += dt * ctl->area;
@@ -2174,21 +2227,11 @@ __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, i
   ctl->sum_kGauss += dt * ctl->kGauss;
   ctl->sum_kMean += dt * ctl->kMean;
   if (sc.cavity_contact) {
-    ctl->sum_pcav += dt * ctl->cavity_force / cavity_surface(ctl->cav_R, sc.cavity_type);
+    ctl->sum_pcav += dt * ctl->cavity_force / cavity_surface(end_step ? ctl->cav_R : ctl->cav_Rm, sc.cavity_type);
     ctl->sum_Nc_cav += dt * (double)ctl->Nc_cav;
     ctl->sum_Ecav += dt * ctl->Ecav;
   }
-  const int pr = ctl->problem;
-  if (pr > ctl->worst_problem) ctl->worst_problem = pr;
-  if (pr > 0 && ctl->first_problem_step == 0) ctl->first_problem_step = ctl->time_step;
-  ctl->steps_done += 1;
-  if (pr >= SHL_STOP_SIM || (sc.stop_on_problem && pr > 0) || ctl->error) ctl->halted = 1;
-  ctl->problem = 0;
-  // the next step's dt, after the measurement used this one (ShellSystem.C:1096-1098)
-  if (sc.adapt_every) set_newmark(ctl, sc, ctl->new_dt);
-  if (ctl->steps_done >= ctl->steps_target) ctl->paused |= 1u;
-  // stopping criterion, tested before the next step (shell.C:314-318)
-  if (sc.sfun_len > 0 && eval_program(sc.sfun, sc.sfun_len, ctl->time, 0.0) != 0.0) ctl->paused |= 2u;
+  if (end_step) end_step_scalar(ctl, sc);
 }
 
 // ------------------------------------------------------------ utilities --
@@ -2403,15 +2446,15 @@ void launch_contact_force(const DevBuf& b, const StepConst& sc, int, cudaStream_
 // mode 2: an adaptive attempt (a_pred and the error estimate); else correct ? step corrector : evaluation
 void launch_gather_correct(const DevBuf& b, const StepConst& sc, int mode, bool correct, double* f_out, double* a_out,
                            cudaStream_t s, RebuildCond rc) {
-  const int m = (mode == 2 || mode == 3) ? mode : (correct ? 1 : 0);
+  const int m = mode >= 2 ? mode : (correct ? 1 : 0);
   k_gather_correct<<<nblk(sc.V), kBlock, 0, s>>>(b, sc, m, f_out, a_out, rc);
 }
 void launch_correct_adapt(const DevBuf& b, const StepConst& sc, cudaStream_t s, RebuildCond rc) {
   k_correct_adapt<<<(sc.V + kBlock - 1) / kBlock, kBlock, 0, s>>>(b, sc, rc);
 }
 
-void launch_volume_end_step(const DevBuf& b, const StepConst& sc, bool end_step, cudaStream_t s) {
-  k_volume_end<<<nblk(sc.F), kBlock, 0, s>>>(b, sc, end_step ? 1 : 0);
+void launch_volume_end_step(const DevBuf& b, const StepConst& sc, int mode, cudaStream_t s) {
+  k_volume_end<<<nblk(sc.F), kBlock, 0, s>>>(b, sc, mode);
 }
 
 // ================================================================ no-alloc --
