@@ -762,7 +762,7 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
     }
     c->blocks_bs[k] = nb ? nb : 1;
   }
-  const uint32_t max_blocks = std::max({blocks, (F + kBlock - 1) / kBlock, (V + kBlock - 1) / kBlock, 4u * 152u}) + 8;
+  const uint32_t max_blocks = std::max({blocks, (F + kBlock - 1) / kBlock, (V + kBlock - 1) / kBlock, 6u * 152u}) + 8;
   ALLOC(b.partial, 8 * (size_t)max_blocks);
   ALLOC(b.partial_v, 8 * (size_t)max_blocks);
   ALLOC(c->d_fa, 2 * nd);

@@ -1774,6 +1774,54 @@ __device__ void cavity_totals(const DevBuf& b, const StepConst& sc, Ctl* ctl, do
   __syncthreads();
 }
 
+// The corrector's last block: maxima and kinetic energy over the blocks'
+// partials, check_increment(true), and what follows from them for the linked
+// cells and the next step.
+__device__ void corrector_scalars(const DevBuf& b, const StepConst& sc, const RebuildCond& rc, int mode) {
+  Ctl* ctl = b.ctl;
+  __shared__ double sh[kBlock / 32];
+  double mm = 0.0, mmn = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+    mm = fmax(mm, __ldcg(&b.partial[(size_t)k * 8]));
+    mmn = fmax(mmn, __ldcg(&b.partial[(size_t)k * 8 + 6]));
+  }
+  mm = block_max(mm, sh);
+  if (mode >= 3) mmn = block_max(mmn, sh);
+  const double ekt = sum_partials(b.partial, 1, gridDim.x, sh);
+  if (sc.n_cs) {  // a batch: each shell's own check_increment(true)
+    if (threadIdx.x == 0) {
+      ctl->Ekin = ekt;
+      if (!isfinite(ekt)) register_problem(ctl, SHL_NOT_FINITE);
+    }
+    batch_correct_check(b, sc, rc, mode >= 3);
+    if (mode >= 4) end_and_begin(b, sc, rc, mode == 4);
+    return;
+  }
+  if (threadIdx.x != 0) return;
+  ctl->Ekin = ekt;
+  if (mode >= 3) ctl->du2_pred = mmn;  // check_increment(false) of the next step, in k_begin_step
+  // check_increment(true)
+  const double du_max = sqrt(mm);
+  if (isfinite(du_max)) {
+    ctl->du_sum = __dadd_rn(ctl->du_sum, __dmul_rn(2.0, du_max));
+    if (du_max == 0.0)
+      register_problem(ctl, SHL_NO_DISP_CHANGE);
+    else if (sc.contact && du_max > 0.5 * sc.thickness)
+      register_problem(ctl, SHL_LARGE_DISP);
+  } else {
+    register_problem(ctl, SHL_NOT_FINITE);
+  }
+  if (!isfinite(ekt)) register_problem(ctl, SHL_NOT_FINITE);
+  const uint32_t flag = (sc.contact && ctl->du_sum >= rebuild_tolerance(sc, ctl)) ? 1u : 0u;
+  if (mode >= 3) {
+    ctl->rebuild_pending = flag;  // made by the next step's IF node, before its own pass
+    if (mode >= 4) end_and_begin(b, sc, rc, mode == 4);
+    return;
+  }
+  ctl->rebuild = flag;
+  set_rebuild_cond(rc, ctl);
+}
+
 __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst sc, int mode, double* f_out,
                                                            double* a_out, RebuildCond rc) {
   // mode 0: eval (write f_out / a_out), mode 1: step corrector, mode 2: adaptive
@@ -2064,46 +2112,187 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
   }
   if (!last_block(&ctl->cnt[3])) return;
   if (sc.cavity_contact) cavity_totals(b, sc, ctl, sh);
-  double mm = 0.0, mmn = 0.0;
-  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-    mm = fmax(mm, __ldcg(&b.partial[(size_t)k * 8]));
-    mmn = fmax(mmn, __ldcg(&b.partial[(size_t)k * 8 + 6]));
-  }
-  mm = block_max(mm, sh);
-  if (mode >= 3) mmn = block_max(mmn, sh);
-  const double ekt = sum_partials(b.partial, 1, gridDim.x, sh);
-  if (sc.n_cs) {  // a batch: each shell's own check_increment(true)
-    if (threadIdx.x == 0) {
-      ctl->Ekin = ekt;
-      if (!isfinite(ekt)) register_problem(ctl, SHL_NOT_FINITE);
+  corrector_scalars(b, sc, rc, mode);
+}
+
+// ---- gather + correct with a node's three components on three lanes ----
+// A thread per node left a level-6 shell (41 k nodes) at 8 warps per SM, each a
+// chain of strided share loads (32 cache lines per load instruction) and FP64
+// operations: 29 us cold.  Here lane 3 i + c of a warp holds component c of its node i
+// (ten nodes per warp): three times the warps, a third of the chain, and a node's
+// share is one 24-byte piece of a cache line per load: 20 us (1.2 M nodes in FP32
+// 300 -> 208, 642 nodes 20 -> 16).  The FP64 pipe (16 cycles
+// per warp instruction) sets the pace, so maxima are taken on the bits and the
+// kinetic energy is summed once per block.  Every per-component operation and
+// the order of every sum is that of k_gather_correct, which stays for cavity
+// contact (its per-node scalar work would be repeated on three lanes) and for the
+// adaptive attempt's norms.
+constexpr int kNodeLanes = 3, kNodesPerWarp = 10, kGatherChunk = kNodesPerWarp * (kBlock / 32);
+constexpr uint32_t kGatherBlocks = 152 * 6;  // a block takes every gridDim.x-th chunk of 80 nodes
+
+// bits of max(x, 0) without NaNs: non-negative doubles compare as integers
+__device__ __forceinline__ unsigned long long max_bits(double x) {
+  return isnan(x) ? 0ull : (unsigned long long)__double_as_longlong(x);
+}
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long x) {
+  const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(x >> 32));
+  const uint32_t lo = __reduce_max_sync(0xffffffffu, (uint32_t)(x >> 32) == hi ? (uint32_t)x : 0u);
+  return (unsigned long long)hi << 32 | lo;
+}
+
+__global__ void __launch_bounds__(kBlock) k_gather_lanes(DevBuf b, StepConst sc, int mode, double* f_out, double* a_out,
+                                                         RebuildCond rc) {
+  // modes as in k_gather_correct (not 2)
+  Ctl* ctl = b.ctl;
+  if (inactive(ctl)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (mode >= 4) ctl->measure = 0u;
+      set_rebuild_cond(rc, ctl);
     }
-    batch_correct_check(b, sc, rc, mode >= 3);
-    if (mode >= 4) end_and_begin(b, sc, rc, mode == 4);
     return;
   }
-  if (threadIdx.x != 0) return;
-  ctl->Ekin = ekt;
-  if (mode >= 3) ctl->du2_pred = mmn;  // check_increment(false) of the next step, in k_begin_step
-  // check_increment(true)
-  const double du_max = sqrt(mm);
-  if (isfinite(du_max)) {
-    ctl->du_sum = __dadd_rn(ctl->du_sum, __dmul_rn(2.0, du_max));
-    if (du_max == 0.0)
-      register_problem(ctl, SHL_NO_DISP_CHANGE);
-    else if (sc.contact && du_max > 0.5 * sc.thickness)
-      register_problem(ctl, SHL_LARGE_DISP);
-  } else {
-    register_problem(ctl, SHL_NOT_FINITE);
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const int c = (int)(lane % 3u), base = (int)lane - c;
+  const bool on_lane = lane < kNodeLanes * kNodesPerWarp;
+  const bool corr = mode == 1 || mode >= 3;
+  unsigned long long du2_max = 0ull, next_max = 0ull;
+  double ekin = 0.0;  // this lane's share over its nodes
+  for (uint32_t n0 = blockIdx.x * kGatherChunk + warp * kNodesPerWarp; n0 < sc.V; n0 += gridDim.x * kGatherChunk) {
+    const uint32_t n = n0 + lane / 3u;
+    const bool on = on_lane && n < sc.V;
+    const size_t k = 3 * (size_t)(on ? n : n0) + c;
+    // the node's state, loaded ahead of (and independently of) the share sums
+    const double vp = b.vp[k], minv = b.Minv[k], damp = b.C[k];
+    const double s_up = corr ? b.up[k] : 0.0, s_u = corr ? b.u[k] : 0.0, s_x = corr ? b.X[k] : 0.0,
+                 s_m = corr ? b.M[k] : 0.0;
+    double f = 0.0;
+    const uint32_t nn = on ? n : n0;
+    if (sc.contact) {
+      const uint32_t k1 = b.csr_ptr[nn + 1];
+#pragma unroll 4
+      for (uint32_t q = b.csr_ptr[nn]; q < k1; ++q) {
+        const uint32_t ent = b.csr_ent[q];
+        const uint32_t role = ent & 7u;
+        const int e = role >= 3 ? 1 : 0, kk = (int)role - 3 * e;
+        const double* pf = b.pforce + kPairOut * (size_t)(ent >> 3);
+        const double vv = pf[3 + 2 * e], ww = pf[4 + 2 * e];
+        const double bary = kk == 0 ? (1.0 - vv - ww) : (kk == 1 ? vv : ww);
+        f += bary * ((e == 0 ? -0.5 : 0.5) * pf[c]);
+      }
+    }
+    const uint32_t g0 = b.gather_ptr[nn], g1 = b.gather_ptr[nn + 1];
+    if (sc.fp32) {
+      float s0 = 0.f;
+      const float* q = b.qe32 + c;
+#pragma unroll 8
+      for (uint32_t j = g0; j < g1; ++j) s0 += q[3 * (size_t)j];
+      f -= (double)s0;
+    } else if (sc.qe_df) {
+      // double-float shares: added as pairs on the FP32 pipe, converted once
+      const float2* q = reinterpret_cast<const float2*>(b.qe) + c;
+      df2 s0 = dfv(0.f);
+#pragma unroll 8
+      for (uint32_t j = g0; j < g1; ++j) {
+        const float2 x = q[3 * (size_t)j];
+        s0 += df2{x.x, x.y};
+      }
+      f -= df_to_double(s0);
+    } else {
+      const double* q = b.qe + c;
+#pragma unroll 8
+      for (uint32_t j = g0; j < g1; ++j) f -= q[3 * (size_t)j];
+    }
+    if (mode >= 1 && b.fcorr) f += b.fcorr[k];  // FP64 defect of the FP32 force (shl_residual)
+    const double ap = minv * (f - damp * vp);
+    if (mode == 0) {
+      if (on) {
+        if (f_out) f_out[k] = f;
+        if (a_out) a_out[k] = ap;
+      }
+      continue;
+    }
+    double un, vn;
+    if (sc.contact) {
+      un = __dadd_rn(__dmul_rn(sc.nm0, ap), s_up);
+      vn = __dadd_rn(__dmul_rn(sc.nm7, ap), vp);
+    } else {
+      un = fma(sc.nm0, ap, s_up);
+      vn = fma(sc.nm7, ap, vp);
+    }
+    const double d = __dsub_rn(un, s_u);
+    const double d0 = __shfl_sync(0xffffffffu, d, base), d1 = __shfl_sync(0xffffffffu, d, base + 1),
+                 d2 = __shfl_sync(0xffffffffu, d, base + 2);
+    const double du2 = d0 * d0 + d1 * d1 + d2 * d2;
+    du2_max = on ? max(du2_max, max_bits(du2)) : du2_max;
+    if (on) ekin = fma(vn * vn, s_m, ekin);
+    double du2_next = 0.0;
+    if (mode >= 3) {
+      // the next step's prediction (predict_node)
+      double up, vp1;
+      if (sc.contact) {
+        up = __dadd_rn(__dmul_rn(sc.dt, vn), un);
+        up = __dadd_rn(__dmul_rn(sc.nm8, ap), up);
+        vp1 = __dadd_rn(__dmul_rn(sc.nm6, ap), vn);
+      } else {
+        up = fma(sc.nm8, ap, fma(sc.dt, vn, un));
+        vp1 = fma(sc.nm6, ap, vn);
+      }
+      const double e = __dsub_rn(up, un), e2 = __dmul_rn(e, e);
+      du2_next = __dadd_rn(__dadd_rn(__shfl_sync(0xffffffffu, e2, base), __shfl_sync(0xffffffffu, e2, base + 1)),
+                           __shfl_sync(0xffffffffu, e2, base + 2));
+      next_max = on ? max(next_max, max_bits(du2_next)) : next_max;
+      if (on) {
+        b.up[k] = up;
+        b.vp[k] = vp1;
+        b.pn[k] = __dadd_rn(s_x, up);
+        if (sc.fp32) {
+          reinterpret_cast<float*>(b.up32)[4 * (size_t)n + c] = (float)up;
+        } else {
+          float h, l;
+          df_split(up, h, l);
+          reinterpret_cast<float2*>(b.upk)[4 * (size_t)n + c] = make_float2(h, l);
+        }
+      }
+    }
+    if (on) {
+      b.u[k] = un;
+      b.v[k] = vn;
+      b.a[k] = ap;
+      b.p[k] = __dadd_rn(s_x, un);
+    }
+    if (sc.n_cs) {
+      const uint32_t nm = on_lane ? n : 0xffffffffu;
+      shell_max_acc(b, sc, nm, du2, 0);
+      if (mode >= 3) shell_max_acc(b, sc, nm, du2_next, 1);
+    }
   }
-  if (!isfinite(ekt)) register_problem(ctl, SHL_NOT_FINITE);
-  const uint32_t flag = (sc.contact && ctl->du_sum >= rebuild_tolerance(sc, ctl)) ? 1u : 0u;
-  if (mode >= 3) {
-    ctl->rebuild_pending = flag;  // made by the next step's IF node, before its own pass
-    if (mode >= 4) end_and_begin(b, sc, rc, mode == 4);
-    return;
+  if (mode == 0) return;
+  __shared__ unsigned long long sh_max[2][kBlock / 32];
+  __shared__ double sh_ek[kBlock];
+  du2_max = warp_max_bits(du2_max);
+  next_max = warp_max_bits(next_max);
+  sh_ek[threadIdx.x] = 0.5 * ekin;
+  if (lane == 0) {
+    sh_max[0][warp] = du2_max;
+    sh_max[1][warp] = next_max;
   }
-  ctl->rebuild = flag;
-  set_rebuild_cond(rc, ctl);
+  __syncthreads();
+  if (warp == 0) {
+    double ek = sh_ek[lane];
+#pragma unroll
+    for (int q = 1; q < kBlock / 32; ++q) ek += sh_ek[32 * q + lane];
+    for (int o = 16; o > 0; o >>= 1) ek += __shfl_down_sync(0xffffffffu, ek, o);
+    const unsigned long long m = warp_max_bits(lane < kBlock / 32 ? sh_max[0][lane] : 0ull);
+    const unsigned long long mn = warp_max_bits(lane < kBlock / 32 ? sh_max[1][lane] : 0ull);
+    if (lane == 0) {
+      double* pp = b.partial + (size_t)blockIdx.x * 8;
+      pp[0] = __longlong_as_double((long long)m);
+      pp[1] = ek;
+      pp[6] = __longlong_as_double((long long)mn);
+    }
+  }
+  if (!last_block(&ctl->cnt[3])) return;
+  corrector_scalars(b, sc, rc, mode);
 }
 
 // corrector of an accepted adaptive attempt (ShellSystem.C:1046-1101): u, v, a
@@ -2447,7 +2636,12 @@ void launch_contact_force(const DevBuf& b, const StepConst& sc, int, cudaStream_
 void launch_gather_correct(const DevBuf& b, const StepConst& sc, int mode, bool correct, double* f_out, double* a_out,
                            cudaStream_t s, RebuildCond rc) {
   const int m = mode >= 2 ? mode : (correct ? 1 : 0);
-  k_gather_correct<<<nblk(sc.V), kBlock, 0, s>>>(b, sc, m, f_out, a_out, rc);
+  if (sc.cavity_contact || m == 2) {
+    k_gather_correct<<<nblk(sc.V), kBlock, 0, s>>>(b, sc, m, f_out, a_out, rc);
+    return;
+  }
+  const uint32_t nb = std::min((sc.V + kGatherChunk - 1) / kGatherChunk, kGatherBlocks);
+  k_gather_lanes<<<nb, kBlock, 0, s>>>(b, sc, m, f_out, a_out, rc);
 }
 void launch_correct_adapt(const DevBuf& b, const StepConst& sc, cudaStream_t s, RebuildCond rc) {
   k_correct_adapt<<<(sc.V + kBlock - 1) / kBlock, kBlock, 0, s>>>(b, sc, rc);
