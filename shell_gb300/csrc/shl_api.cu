@@ -2126,12 +2126,12 @@ shl_status shl_get_node_fields(shl_ctx* c, double* ekin, double* ecav, double* e
   SHL_CUDA_TRY(cudaStreamSynchronize(c->stream));
   for (uint32_t j = 0; j < np; ++j) {
     const double* o = &pf[(size_t)kPairOut * j];
-    const double es = o[7], ef = o[8];
+    const double es = o[kPairEself], ef = o[kPairEfric];
     if (es == 0.0 && ef == 0.0) continue;
     const uint32_t ee[2] = {e1[j], e2[j]};
     const double area_min = std::min(area[ee[0]], area[ee[1]]);
     for (int s = 0; s < 2; ++s) {
-      const double vv = o[3 + 2 * s], ww = o[4 + 2 * s];
+      const double vv = o[kPairBary + 3 * s + 1], ww = o[kPairBary + 3 * s + 2];
       const double w[3] = {0.5 * (1.0 - vv - ww) / area_min, 0.5 * vv / area_min, 0.5 * ww / area_min};
       for (int k = 0; k < 3; ++k) {
         const uint32_t n = T[3 * (size_t)ee[s] + k];

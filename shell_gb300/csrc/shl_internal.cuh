@@ -32,8 +32,13 @@ namespace shl {
 constexpr int kBlock = 256;          // threads per block for element / node kernels
 constexpr int kMaxGroups = 8;        // patch groups (regular + irregular valences)
 constexpr int kMaxSlots = 18;        // patch slots of the largest supported valence (12)
-// doubles per contact pair written by the contact-force kernel
-constexpr int kPairOut = 9;
+// A contact pair's record, written by the contact-force kernel: half its force
+// (a node's share is -/+ that times its barycentric), the self-contact energy,
+// the barycentrics of the six nodes (element 1, then 2), the friction energy and
+// a pad -- three 32-byte sectors, of which a node reads two.  The gather's loop over
+// a node's contacts is then one fused multiply-add per component.
+constexpr int kPairOut = 12;
+constexpr int kPairEself = 3, kPairBary = 4, kPairEfric = 10;
 constexpr int kScanTile = 2048;      // elements per block in the multi-block scan
 
 // Patch-group description for the element kernel (in __constant__ memory).
@@ -265,7 +270,7 @@ struct DevBuf {
   double* cand_d2;
   uint8_t* cand_ok;
   uint32_t* seg_count;         // per-face pair counts (F)
-  double* pforce;              // kPairOut per pair: f_contact(3), v1, w1, v2, w2, Eself, Efric
+  double* pforce;              // kPairOut per pair
   // SMOOTH contact
   double* pvw[2];              // 4 per pair: the closest-point search's (v1, w1, v2, w2), patch frames
   double* new_x;               // 4 per new pair of a rebuild

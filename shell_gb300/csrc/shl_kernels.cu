@@ -1728,9 +1728,14 @@ __global__ void __launch_bounds__(kBlock) k_contact_force(DevBuf b, StepConst sc
       }
       f_normal = SHL_SUB(f_normal, SHL_MUL(SHL_MUL(sc.self_damping, stiffness), abs_v_normal));
       for (int c = 0; c < 3; ++c) fcon[c] = SHL_ADD(fcon[c], SHL_MUL(f_normal, nrm[c]));
-      out[0] = fcon[0]; out[1] = fcon[1]; out[2] = fcon[2];
-      out[3] = g.v[0]; out[4] = g.w[0]; out[5] = g.v[1]; out[6] = g.w[1];
-      out[7] = es; out[8] = ef;
+      for (int c = 0; c < 3; ++c) out[c] = 0.5 * fcon[c];
+      for (int t = 0; t < 2; ++t) {
+        out[kPairBary + 3 * t] = uu[t];
+        out[kPairBary + 3 * t + 1] = g.v[t];
+        out[kPairBary + 3 * t + 2] = g.w[t];
+      }
+      out[kPairEself] = es;
+      out[kPairEfric] = ef;
     } else {
       b.porig[0][3 * (size_t)j] = 0.0;
       b.porig[0][3 * (size_t)j + 1] = 0.0;
@@ -1864,15 +1869,12 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
 #pragma unroll 4
       for (uint32_t k = k0; k < k1; ++k) {
         const uint32_t ent = b.csr_ent[k];
-        const uint32_t j = ent >> 3, role = ent & 7u;
-        const int e = role >= 3 ? 1 : 0, kk = role - 3 * e;
-        const double* pf = b.pforce + kPairOut * (size_t)j;
-        const double vv = pf[3 + 2 * e], ww = pf[4 + 2 * e];
-        const double bary = kk == 0 ? (1.0 - vv - ww) : (kk == 1 ? vv : ww);
-        const double pref = e == 0 ? -0.5 : 0.5;
-        f[0] += bary * (pref * pf[0]);
-        f[1] += bary * (pref * pf[1]);
-        f[2] += bary * (pref * pf[2]);
+        const uint32_t role = ent & 7u;
+        const double* pf = b.pforce + kPairOut * (size_t)(ent >> 3);
+        const double w = pf[kPairBary + role], bary = role < 3 ? -w : w;
+        f[0] = fma(bary, pf[0], f[0]);
+        f[1] = fma(bary, pf[1], f[1]);
+        f[2] = fma(bary, pf[2], f[2]);
       }
     }
     const uint32_t g0 = b.gather_ptr[n], g1 = b.gather_ptr[n + 1];
@@ -2169,15 +2171,13 @@ __global__ void __launch_bounds__(kBlock) k_gather_lanes(DevBuf b, StepConst sc,
     const uint32_t nn = on ? n : n0;
     if (sc.contact) {
       const uint32_t k1 = b.csr_ptr[nn + 1];
-#pragma unroll 4
+#pragma unroll 8
       for (uint32_t q = b.csr_ptr[nn]; q < k1; ++q) {
         const uint32_t ent = b.csr_ent[q];
         const uint32_t role = ent & 7u;
-        const int e = role >= 3 ? 1 : 0, kk = (int)role - 3 * e;
         const double* pf = b.pforce + kPairOut * (size_t)(ent >> 3);
-        const double vv = pf[3 + 2 * e], ww = pf[4 + 2 * e];
-        const double bary = kk == 0 ? (1.0 - vv - ww) : (kk == 1 ? vv : ww);
-        f += bary * ((e == 0 ? -0.5 : 0.5) * pf[c]);
+        const double w = pf[kPairBary + role];
+        f = fma(role < 3 ? -w : w, pf[c], f);
       }
     }
     const uint32_t g0 = b.gather_ptr[nn], g1 = b.gather_ptr[nn + 1];
