@@ -349,7 +349,8 @@ __device__ __forceinline__ CavityGeom cavity_geom(const double* R, const StepCon
 }
 
 // cavity surface (Knud Thomsen's approximation for the ellipsoid, an ellipse
-// circumference approximation for the cylinder), ShellSystem.C:441-468
+// circumference approximation for the cylinder), ShellSystem.C:441-468.  Called
+// by one warp; the ellipsoid's three powers are taken by three lanes.
 __device__ double cavity_surface(const double* R, int type) {
   const double Rx = R[0], Ry = R[1], Rz = R[2];
   if (type == SHL_CAVITY_BOX) return 8 * (Rx * Ry + Rx * Rz + Ry * Rz);
@@ -358,8 +359,11 @@ __device__ double cavity_surface(const double* R, int type) {
     const double lambda32 = 3 * lambda * lambda;
     return 2 * 3.141592653589793238 * ((Ry + Rz) * (1 + lambda32 / (10 + sqrt(4 - lambda32))) + Ry * Rz);
   }
-  return 4 * 3.141592653589793238 *
-         pow((pow(Rx * Ry, 1.6) + pow(Rx * Rz, 1.6) + pow(Ry * Rz, 1.6)) / 3, 0.625);
+  const uint32_t lane = threadIdx.x & 31u;
+  const double p = pow(lane == 0 ? Rx * Ry : (lane == 1 ? Rx * Rz : Ry * Rz), 1.6);
+  const double p0 = __shfl_sync(0xffffffffu, p, 0), p1 = __shfl_sync(0xffffffffu, p, 1),
+               p2 = __shfl_sync(0xffffffffu, p, 2);
+  return 4 * 3.141592653589793238 * pow((p0 + p1 + p2) / 3, 0.625);
 }
 
 // ------------------------------------------------ config expressions --
@@ -2409,6 +2413,12 @@ __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, i
     for (int k = 0; k < 6; ++k) pp[k] = v[k];
   }
   if (!last_block(&ctl->cnt[4])) return;
+  // the cavity's surface on a warp that has no column to sum, beside the sums
+  __shared__ double surface;
+  if (sc.cavity_contact && mode != kVolTotals && threadIdx.x >= kBlock - 32) {
+    const double x = cavity_surface(end_step ? ctl->cav_R : ctl->cav_Rm, sc.cavity_type);
+    if (threadIdx.x == kBlock - 32) surface = x;
+  }
   double t[6];
   sum_partials_t<6>(b.partial_v, gridDim.x, sh, t);
   if (threadIdx.x != 0) return;
@@ -2428,7 +2438,7 @@ __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, i
   ctl->sum_kGauss += dt * ctl->kGauss;
   ctl->sum_kMean += dt * ctl->kMean;
   if (sc.cavity_contact) {
-    ctl->sum_pcav += dt * ctl->cavity_force / cavity_surface(end_step ? ctl->cav_R : ctl->cav_Rm, sc.cavity_type);
+    ctl->sum_pcav += dt * ctl->cavity_force / surface;
     ctl->sum_Nc_cav += dt * (double)ctl->Nc_cav;
     ctl->sum_Ecav += dt * ctl->Ecav;
   }
@@ -2648,7 +2658,12 @@ void launch_gather_correct(const DevBuf& b, const StepConst& sc, int mode, bool 
                            cudaStream_t s, RebuildCond rc) {
   const int m = mode >= 2 ? mode : (correct ? 1 : 0);
   if (sc.cavity_contact || m == 2) {
-    k_gather_correct<<<nblk(sc.V), kBlock, 0, s>>>(b, sc, m, f_out, a_out, rc);
+    // the cavity's geometry is some 400 FP64 operations per node: small shells
+    // take smaller blocks, so that all SMs' FP64 pipes share them (4,412 nodes:
+    // 18 blocks of 256 took 35 us warm, 138 of 32 take 23)
+    uint32_t bs = kBlock;
+    while (bs > 32 && sc.V <= 152u * (bs / 2)) bs /= 2;
+    k_gather_correct<<<(sc.V + bs - 1) / bs, bs, 0, s>>>(b, sc, m, f_out, a_out, rc);
     return;
   }
   const uint32_t nb = std::min((sc.V + kGatherChunk - 1) / kGatherChunk, kGatherBlocks);
