@@ -455,97 +455,103 @@ __global__ void __launch_bounds__(kBlock) k_rb_count(DevBuf b, StepConst sc) {
 
 // ----------------------------------------------------------------- scan --
 // Exclusive scan of in[0..n) into out[0..n) (+ out[n] = total if with_end),
-// gated by *gate; two launches, fixed grids sized by capacity.
+// gated by *gate; two launches.  n may be far below its capacity (the cells of a
+// batch of which one shell is rebuilt; no pass at all), so the blocks are at most
+// kScanBlocks and take every gridDim.x-th tile (a block per tile of the capacity:
+// 68 us for the 100,000 tiles of a 256-shell batch that had nothing to scan).
+constexpr uint32_t kScanBlocks = 152 * 8;
 __global__ void __launch_bounds__(kBlock) k_scan_tiles(const uint32_t* gate, const Ctl* ctl, const uint32_t* in,
                                                        uint32_t* out, const uint32_t* n_ptr, uint32_t n_const,
                                                        uint32_t* tile_sums) {
   if (*gate == 0 || ctl->halted) return;
   const uint32_t n = n_ptr ? *n_ptr : n_const;
-  const uint32_t base = blockIdx.x * kScanTile;
-  if (base >= n) return;
   constexpr int PER = kScanTile / kBlock;
-  uint32_t v[PER];
-  uint32_t sum = 0;
-  const uint32_t i0 = base + threadIdx.x * PER;
-#pragma unroll
-  for (int k = 0; k < PER; ++k) {
-    const uint32_t x = (i0 + k < n) ? in[i0 + k] : 0u;
-    v[k] = sum;
-    sum += x;
-  }
-  // exclusive scan of the per-thread sums over the block
   __shared__ uint32_t wsum[kBlock / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t incl = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) wsum[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t w = (lane < kBlock / 32) ? wsum[lane] : 0u;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    if (lane < kBlock / 32) wsum[lane] = w;
-  }
-  __syncthreads();
-  const uint32_t excl = incl - sum + (warp > 0 ? wsum[warp - 1] : 0u);
+  for (uint32_t tile = blockIdx.x; (uint64_t)tile * kScanTile < n; tile += gridDim.x) {
+    uint32_t v[PER];
+    uint32_t sum = 0;
+    const uint32_t i0 = tile * kScanTile + threadIdx.x * PER;
 #pragma unroll
-  for (int k = 0; k < PER; ++k)
-    if (i0 + k < n) out[i0 + k] = v[k] + excl;
-  if (threadIdx.x == kBlock - 1) tile_sums[blockIdx.x] = excl + sum;
+    for (int k = 0; k < PER; ++k) {
+      const uint32_t x = (i0 + k < n) ? in[i0 + k] : 0u;
+      v[k] = sum;
+      sum += x;
+    }
+    // exclusive scan of the per-thread sums over the block
+    uint32_t incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    __syncthreads();  // the previous tile's sums have been read
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t w = (lane < kBlock / 32) ? wsum[lane] : 0u;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+      }
+      if (lane < kBlock / 32) wsum[lane] = w;
+    }
+    __syncthreads();
+    const uint32_t excl = incl - sum + (warp > 0 ? wsum[warp - 1] : 0u);
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+      if (i0 + k < n) out[i0 + k] = v[k] + excl;
+    if (threadIdx.x == kBlock - 1) tile_sums[tile] = excl + sum;
+  }
 }
 
-// Each tile's offset is the sum of the tiles before it, added up by the tile's
-// own block (a few hundred tile sums at most); block 0 adds all of them: the
-// total, out[n] and the capacity check.
+// Each tile's offset is the sum of the tiles before it, added up by the block that
+// takes the tile (from its previous tile on); block 0 adds all of them: the total,
+// out[n] and the capacity check.
 __global__ void __launch_bounds__(kBlock) k_scan_add(const uint32_t* gate, Ctl* ctl, uint32_t* out,
                                                      const uint32_t* n_ptr, uint32_t n_const,
                                                      const uint32_t* tile_sums, uint32_t* total, int with_end,
                                                      uint32_t cap, int cap_error) {
   if (*gate == 0 || ctl->halted) return;
   const uint32_t n = n_ptr ? *n_ptr : n_const;
-  const uint32_t base = blockIdx.x * kScanTile;
-  if (blockIdx.x != 0 && base >= n) return;
-  const uint32_t upto = blockIdx.x == 0 ? (n + kScanTile - 1) / kScanTile : blockIdx.x;
-  uint32_t s = 0;
-  for (uint32_t t = threadIdx.x; t < upto; t += blockDim.x) s += tile_sums[t];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   __shared__ uint32_t wsum[kBlock / 32];
-  __shared__ uint32_t offset;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) wsum[warp] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < kBlock / 32; ++w) t += wsum[w];
-    offset = t;
+  // the block's sum of tile_sums[from, to), in every thread
+  auto block_total = [&](uint32_t from, uint32_t to) {
+    uint32_t s = 0;
+    for (uint32_t t = from + threadIdx.x; t < to; t += blockDim.x) s += tile_sums[t];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    __syncthreads();
+    if (lane == 0) wsum[warp] = s;
+    __syncthreads();
+    s = 0;
+    for (int w = 0; w < kBlock / 32; ++w) s += wsum[w];
+    return s;
+  };
+  uint32_t add = 0, done = 0;  // the offset of tile `done`
+  for (uint32_t tile = blockIdx.x; (uint64_t)tile * kScanTile < n; tile += gridDim.x) {
+    add += block_total(done, tile);
+    done = tile;
+    if (tile == 0) continue;
+    const uint32_t base = tile * kScanTile;
+    for (uint32_t i = base + threadIdx.x; i < base + kScanTile && i < n; i += blockDim.x) out[i] += add;
   }
-  __syncthreads();
-  const uint32_t add = offset;
-  if (blockIdx.x == 0) {
-    if (threadIdx.x == 0) {
-      *total = add;
-      if (with_end) out[n] = add;
-      if (cap_error && add > cap) {
-        atomicMax(&ctl->error, (int)SHL_ERR_CAPACITY);
-        ctl->rebuild = 0;
-        ctl->csr_dirty = 0;
-      }
-    }
-    return;
+  if (blockIdx.x != 0) return;
+  add += block_total(done, (n + kScanTile - 1) / kScanTile);
+  if (threadIdx.x != 0) return;
+  *total = add;
+  if (with_end) out[n] = add;
+  if (cap_error && add > cap) {
+    atomicMax(&ctl->error, (int)SHL_ERR_CAPACITY);
+    ctl->rebuild = 0;
+    ctl->csr_dirty = 0;
   }
-  for (uint32_t i = base + threadIdx.x; i < base + kScanTile && i < n; i += blockDim.x) out[i] += add;
 }
 
 void launch_scan(const uint32_t* gate, Ctl* ctl, const uint32_t* in, uint32_t* out, const uint32_t* n_ptr,
                  uint32_t n_const, uint32_t n_cap, uint32_t* tile_sums, uint32_t* total, bool with_end,
                  uint32_t cap, bool cap_error, cudaStream_t s) {
   const uint32_t nt = (n_cap + kScanTile - 1) / kScanTile;
-  const uint32_t grid = nt > 0 ? nt : 1;
+  const uint32_t grid = std::min(nt > 0 ? nt : 1u, kScanBlocks);
   k_scan_tiles<<<grid, kBlock, 0, s>>>(gate, ctl, in, out, n_ptr, n_const, tile_sums);
   k_scan_add<<<grid, kBlock, 0, s>>>(gate, ctl, out, n_ptr, n_const, tile_sums, total, with_end ? 1 : 0, cap,
                                      cap_error ? 1 : 0);
@@ -1442,26 +1448,29 @@ __global__ void __launch_bounds__(32 * kCsrSortWarps) k_csr_sort(DevBuf b, StepC
   Ctl* ctl = b.ctl;
   if (csr_off(ctl)) return;
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint32_t me = (blockIdx.x * kCsrSortWarps + w) * kCsrSortNodes + lane;
-  uint32_t k0 = 0, n = 0;
-  if (lane < kCsrSortNodes && me < sc.V) {
-    k0 = b.csr_ptr[me];
-    n = b.csr_ptr[me + 1] - k0;
-  }
-  // larger segments than the registers hold go to the list of k_csr_sort_big
-  if (n > kCsrSortCap) b.csr_fill[atomicAdd(&ctl->cnt[9], 1u)] = me;
-  unsigned todo = __ballot_sync(0xffffffffu, n >= 2 && n <= kCsrSortCap);
-  while (todo) {
-    const int src = __ffs(todo) - 1;
-    todo &= todo - 1;
-    uint32_t* ent = b.csr_ent + __shfl_sync(0xffffffffu, k0, src);
-    const uint32_t sn = __shfl_sync(0xffffffffu, n, src);
-    if (sn <= 32) warp_sort_segment<1>(ent, sn);
-    else if (sn <= 64) warp_sort_segment<2>(ent, sn);
-    else if (sn <= 128) warp_sort_segment<4>(ent, sn);
-    else if (sn <= 256) warp_sort_segment<8>(ent, sn);
-    else if (sn <= 512) warp_sort_segment<16>(ent, sn);
-    else warp_sort_segment<32>(ent, sn);
+  for (uint32_t base = (blockIdx.x * kCsrSortWarps + w) * kCsrSortNodes; base < sc.V;
+       base += gridDim.x * kCsrSortWarps * kCsrSortNodes) {
+    const uint32_t me = base + lane;
+    uint32_t k0 = 0, n = 0;
+    if (lane < kCsrSortNodes && me < sc.V) {
+      k0 = b.csr_ptr[me];
+      n = b.csr_ptr[me + 1] - k0;
+    }
+    // larger segments than the registers hold go to the list of k_csr_sort_big
+    if (n > kCsrSortCap) b.csr_fill[atomicAdd(&ctl->cnt[9], 1u)] = me;
+    unsigned todo = __ballot_sync(0xffffffffu, n >= 2 && n <= kCsrSortCap);
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      uint32_t* ent = b.csr_ent + __shfl_sync(0xffffffffu, k0, src);
+      const uint32_t sn = __shfl_sync(0xffffffffu, n, src);
+      if (sn <= 32) warp_sort_segment<1>(ent, sn);
+      else if (sn <= 64) warp_sort_segment<2>(ent, sn);
+      else if (sn <= 128) warp_sort_segment<4>(ent, sn);
+      else if (sn <= 256) warp_sort_segment<8>(ent, sn);
+      else if (sn <= 512) warp_sort_segment<16>(ent, sn);
+      else warp_sort_segment<32>(ent, sn);
+    }
   }
 }
 
@@ -1524,7 +1533,7 @@ void launch_contact_csr(const DevBuf& b, const StepConst& sc, cudaStream_t s) {
               true, sc.csr_cap, true, s);
   k_csr_fill<<<gP, kBlock, 0, s>>>(b, sc);
   {
-    const uint32_t g = (sc.V + kCsrSortNodes * kCsrSortWarps - 1) / (kCsrSortNodes * kCsrSortWarps);
+    const uint32_t g = std::min((sc.V + kCsrSortNodes * kCsrSortWarps - 1) / (kCsrSortNodes * kCsrSortWarps), 16u * 152u);
     k_csr_sort<<<g ? g : 1, 32 * kCsrSortWarps, 0, s>>>(b, sc);
     k_csr_sort_big<<<152, kCsrSortBigBlock, kCsrSortBigCap * 4, s>>>(b, sc);
   }
