@@ -711,7 +711,7 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
   if (fp32) {
     ALLOC(b.qe32, 3 * (size_t)S.n_slots_total);
     ALLOC(b.up32, (size_t)V);
-    ALLOC(b.face32, (size_t)F32_COUNT * F);
+    ALLOC(b.face32, (size_t)kFace32Stride * F);
   } else {
     ALLOC(b.face_df, (size_t)2 * kSplitStride * F);
     if (params->shell_shell_contact == SHL_CONTACT_SMOOTH) ALLOC(b.face_soa, S.face_soa.size());

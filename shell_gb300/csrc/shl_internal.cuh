@@ -231,7 +231,7 @@ struct DevBuf {
   double* pscale;     // F (internal order): factor on the step's pressure (per shell)
   int32_t* patch;     // patch_rows * F, slot-major
   double* qe;         // 3 per element-force slot, in gather order (slot_pos)
-  float* face32;      // F32_COUNT * F (FP32 element path)
+  float* face32;      // kFace32Stride per face (FP32 element path)
   float* face_df;     // kSplitStride float pairs per face (FP64 path: the component-split kernel)
   float* face_soa;    // 2 * F32_COUNT * F: the FP32 constants as float pairs (SMOOTH contact: hi rows, then lo rows)
   int32_t* patch12;   // regular faces: 12 patch node ids per face

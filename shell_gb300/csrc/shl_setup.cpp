@@ -481,14 +481,14 @@ bool build_setup(const shl_mesh& mesh, const shl_params& prm, Setup& S, std::str
     }
   }
   // FP32 constants of the relative-displacement element path
-  S.face32.assign((size_t)F32_COUNT * F, 0.0f);
+  S.face32.assign((size_t)kFace32Stride * F, 0.0f);
   const bool soa = prm.shell_shell_contact == SHL_CONTACT_SMOOTH;
   if (soa) S.face_soa.assign((size_t)2 * F32_COUNT * F, 0.0f);
   for (uint32_t i = 0; i < F; ++i) {
     auto get = [&](int fld) { return face_bal[(size_t)fld * F + i]; };
     auto put32 = [&](int fld, double x) {
       const float h = (float)x;
-      S.face32[(size_t)fld * F + i] = h;
+      S.face32[(size_t)kFace32Stride * i + fld] = h;
       if (!soa) return;
       S.face_soa[(size_t)fld * F + i] = h;
       S.face_soa[(size_t)(F32_COUNT + fld) * F + i] = (float)(x - (double)h);
@@ -672,7 +672,7 @@ bool merge_setups(std::vector<Setup>& shells, Setup& M, std::vector<uint32_t>& n
   layout_slots(M);
   M.patch.assign((size_t)M.patch_rows * F, -1);
   M.face.assign((size_t)FF_COUNT * F, 0.0);
-  M.face32.assign((size_t)F32_COUNT * F, 0.0f);
+  M.face32.assign((size_t)kFace32Stride * F, 0.0f);
   const bool soa = !shells[0].face_soa.empty();
   if (soa) M.face_soa.assign((size_t)2 * F32_COUNT * F, 0.0f);
   M.split.assign((size_t)kSplitStride * F, 0.0);
@@ -684,7 +684,7 @@ bool merge_setups(std::vector<Setup>& shells, Setup& M, std::vector<uint32_t>& n
       M.patch[(size_t)s * F + i] = nd < 0 ? -1 : nd + (int32_t)node_off[k];
     }
     for (int fld = 0; fld < FF_COUNT; ++fld) M.face[(size_t)fld * F + i] = S.face[(size_t)fld * S.F + si];
-    for (int fld = 0; fld < F32_COUNT; ++fld) M.face32[(size_t)fld * F + i] = S.face32[(size_t)fld * S.F + si];
+    std::copy_n(&S.face32[(size_t)kFace32Stride * si], kFace32Stride, &M.face32[(size_t)kFace32Stride * i]);
     if (soa)
       for (int fld = 0; fld < 2 * F32_COUNT; ++fld)
         M.face_soa[(size_t)fld * F + i] = S.face_soa[(size_t)fld * S.F + si];

@@ -40,7 +40,8 @@ enum FaceField {
   FF_COUNT
 };
 
-// Per-face FP32 constants of the FP32 element path (structure of arrays).
+// Per-face FP32 constants of the FP32 element path (one record of kFace32Stride
+// floats per face).
 // The strains are formed from the displacement relative to this reference
 // geometry, so no difference of nearly equal metrics is taken.
 enum FaceField32 {
@@ -54,6 +55,9 @@ enum FaceField32 {
   F32_K, F32_D,
   F32_COUNT
 };
+
+constexpr int kFace32Stride = 40;  // floats per record: ten 16-byte pieces
+static_assert(F32_COUNT <= kFace32Stride, "record size");
 
 // Per-face constants of the component-split element kernel (one record of
 // kSplitStride values per face, internal order): the balanced material frame
@@ -100,7 +104,7 @@ struct Setup {
   uint32_t n_slots_total = 0;      // element-force slots of all faces (sum of n_slots)
   std::vector<int32_t> patch;      // [slot * F + internal face], -1 for unused slots
   std::vector<double> face;        // [field * F + internal face]
-  std::vector<float> face32;       // [FaceField32 * F + internal face]
+  std::vector<float> face32;       // [internal face * kFace32Stride + FaceField32]
   std::vector<float> face_soa;     // SMOOTH contact: the same as float pairs, hi [fld * F + i], lo [(F32_COUNT + fld) * F + i]
   std::vector<double> split;       // [internal face * kSplitStride + SplitField]
   std::vector<double> Minv, C;     // 3V node-major
