@@ -252,7 +252,7 @@ struct DevBuf {
   uint32_t *close_ptr, *close_list;
   // contact: per-face AABB (original order), size, cell ranges
   double *bmin, *bmax, *fsize;
-  int32_t *cell_lo, *cell_hi;  // 3 per face
+  int32_t *cell_lo, *cell_hi;  // cell ranges: lowest cell, 4 per face (one 16-byte load), highest, 3 per face
   uint32_t *cell_count, *cell_start, *cell_fill, *cell_items;
   uint32_t* scan_block;        // block sums for the scans
   // pair lists (double buffered: cur / old), sorted by (e1, e2)
