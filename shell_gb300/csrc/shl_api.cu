@@ -178,7 +178,7 @@ void split_to_soa(const Setup& S, std::vector<float>& out) {
         out[(size_t)fld * S.F + i] = h;
         out[(size_t)(F32_COUNT + fld) * S.F + i] = (float)(x - (double)h);
       };
-      for (int k = 0; k < 4; ++k) put(F32_R00 + k, r[SF_R00 + k] * (g.valence == 6 ? 324.0 : 1.0));
+      for (int k = 0; k < 4; ++k) put(F32_R00 + k, r[SF_R00 + k] * (g.valence == 6 ? kSplitDen1 : 1.0));
       for (const auto& m : map) put(m[0], r[m[1]]);
       for (const auto& v : vec)
         for (int k = 0; k < 3; ++k) put(v[0] + k, r[v[1] + k]);

@@ -518,7 +518,7 @@ bool build_setup(const shl_mesh& mesh, const shl_params& prm, Setup& S, std::str
     for (uint32_t i = g.first; i < g.first + g.count; ++i) {
       auto get = [&](int fld) { return face_bal[(size_t)fld * F + i]; };
       double* r = &S.split[(size_t)kSplitStride * i];
-      const double q1 = g.valence == 6 ? 324.0 : 1.0, q2 = g.valence == 6 ? 108.0 : 1.0;
+      const double q1 = g.valence == 6 ? kSplitDen1 : 1.0, q2 = g.valence == 6 ? kSplitDen2 : 1.0;
       const double R00 = get(FF_R00), R01 = get(FF_R01), R10 = get(FF_R10), R11 = get(FF_R11);
       r[SF_R00] = R00 / q1; r[SF_R01] = R01 / q1; r[SF_R10] = R10 / q1; r[SF_R11] = R11 / q1;
       r[SF_C11A] = R00 * R00 / q2; r[SF_C11B] = R10 * R10 / q2; r[SF_C11C] = 2 * R00 * R10 / q2;

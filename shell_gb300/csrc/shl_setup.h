@@ -63,7 +63,7 @@ static_assert(F32_COUNT <= kFace32Stride, "record size");
 // kSplitStride values per face, internal order): the balanced material frame
 // (|k| = |j| = sqrt |b1 x b2|; reinit_mod's scaling degenerates on some faces).
 // On a regular patch R and the second-derivative coefficients C are divided by
-// the denominators of the basis derivatives (324 and 108).
+// the denominators of the basis derivatives.
 enum SplitField {
   SF_R00, SF_R01, SF_R10, SF_R11,  // rotation onto the material frame
   SF_C11A, SF_C11B, SF_C11C,       // R00^2, R10^2, 2 R00 R10
@@ -80,6 +80,7 @@ enum SplitField {
   SF_K = SF_H + 6, SF_D,
   SF_COUNT
 };
+constexpr double kSplitDen1 = 162.0, kSplitDen2 = 18.0;  // SHL_REGULAR_BASIS
 constexpr int kSplitStride = 52;   // values per record: a multiple of 16 bytes as float pairs
 static_assert(SF_COUNT <= kSplitStride, "record size");
 

@@ -12,7 +12,9 @@
 // stress resultants is one lane's.  The chain is a third as long and needs 96
 // registers, so that twice the warps share an SM.  Cold, in us: 1,280 faces
 // 59 -> 30, 81,920 faces 77 -> 56, 163,840 faces 132 -> 84 (warm, 8,820 faces
-// 34 -> 15).  Bound by FP32 issue at the large end and by the chain at the small.
+// 34 -> 15).  Summing products in one accumulator, exact power-of-two weights and
+// sums made by one lane for all three took 163,840 faces from 84 to 72.  Bound by
+// FP32 issue at the large end (64 % of the slots) and by the chain at the small.
 //
 // The mechanics are those of the relative-displacement form: no step subtracts
 // nearly equal quantities.
@@ -39,12 +41,13 @@
 namespace shl {
 
 // basis (phi, d/dv, d/dw, d2/dv2, d2/dw2, d2/dvdw) of a regular patch's slots at
-// the centroid, times 972, 324, 324, 108, 108, 108
+// the centroid, times 972, 162, 162, 18, 18, 18 (kSplitDen1, kSplitDen2: most of
+// the derivatives are powers of two)
 #define SHL_REGULAR_BASIS { \
-    {276, -156, -156, -24, -24, 24}, {276, 156, 0, -24, -96, -48}, {276, 0, 156, -96, -24, -48}, \
-    {42, -60, 0, 48, -24, -12},      {3, -10, -8, 24, 12, 18},     {3, -8, -10, 12, 24, 18}, \
-    {42, 0, -60, -24, 48, -12},      {42, 60, 60, 48, 48, 60},     {3, 10, 2, 24, 0, 6}, \
-    {3, 8, -2, 12, 0, -6},           {3, 2, 10, 0, 24, 6},         {3, -2, 8, 0, 12, -6}}
+    {276, -78, -78, -4, -4, 4}, {276, 78, 0, -4, -16, -8}, {276, 0, 78, -16, -4, -8}, \
+    {42, -30, 0, 8, -4, -2},    {3, -5, -4, 4, 2, 3},      {3, -4, -5, 2, 4, 3}, \
+    {42, 0, -30, -4, 8, -2},    {42, 30, 30, 8, 8, 10},    {3, 5, 1, 4, 0, 1}, \
+    {3, 4, -1, 2, 0, -1},       {3, 1, 5, 0, 4, 1},        {3, -1, 4, 0, 2, -1}}
 
 static_assert(kSplitFaces * 3 <= 32, "three lanes per face (lanes 30 and 31 repeat the last face)");
 
@@ -53,7 +56,8 @@ __device__ __forceinline__ df2 lane_of(df2 x, int src) {
   return {__shfl_sync(0xffffffffu, x.h, src), __shfl_sync(0xffffffffu, x.l, src)};
 }
 
-// a sum of weight * value terms
+// a sum of products; its terms' errors go to l, normalised once at the end (a
+// product and its sum cost 12 instructions, where df2's operators take 18)
 struct Acc {
   float h = 0.f, l = 0.f;
   __device__ __forceinline__ void first(float w, df2 x) {
@@ -75,12 +79,64 @@ struct Acc {
     const float p = __fmul_rn(w.x, x.h);
     two_sum(p, __fmaf_rn(w.y, x.h, __fmaf_rn(w.x, x.l, __fmaf_rn(w.x, x.h, -p))));
   }
+  // w a power of two: the product is exact
+  __device__ __forceinline__ void first_exact(float w, df2 x) {
+    h = __fmul_rn(w, x.h);
+    l = __fmul_rn(w, x.l);
+  }
+  __device__ __forceinline__ void add_exact(float w, df2 x) {
+    const float s = __fmaf_rn(w, x.h, h);
+    const float bb = __fsub_rn(s, h);
+    const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fmaf_rn(w, x.h, -bb));
+    l = __fadd_rn(l, __fmaf_rn(w, x.l, err));
+    h = s;
+  }
+  // w a compile-time integer
+  __device__ __forceinline__ void first_int(int w, df2 x) {
+    if ((w & (w - 1)) == 0 || (-w & (-w - 1)) == 0) first_exact((float)w, x);
+    else first((float)w, x);
+  }
+  __device__ __forceinline__ void add_int(int w, df2 x) {
+    if ((w & (w - 1)) == 0 || (-w & (-w - 1)) == 0) add_exact((float)w, x);
+    else add((float)w, x);
+  }
+  __device__ __forceinline__ void first(df2 x, df2 y) {
+    h = __fmul_rn(x.h, y.h);
+    l = __fmaf_rn(x.l, y.h, __fmaf_rn(x.h, y.l, __fmaf_rn(x.h, y.h, -h)));
+  }
+  __device__ __forceinline__ void add(df2 x, df2 y) {
+    const float p = __fmul_rn(x.h, y.h);
+    two_sum(p, __fmaf_rn(x.l, y.h, __fmaf_rn(x.h, y.l, __fmaf_rn(x.h, y.h, -p))));
+  }
   __device__ __forceinline__ df2 value() const {
     df2 r;
     df_quick_two_sum(h, l, r.h, r.l);
     return r;
   }
 };
+
+__device__ __forceinline__ df2 dot2(df2 x0, df2 y0, df2 x1, df2 y1) {
+  Acc a;
+  a.first(x0, y0);
+  a.add(x1, y1);
+  return a.value();
+}
+__device__ __forceinline__ df2 dot3(df2 x0, df2 y0, df2 x1, df2 y1, df2 x2, df2 y2) {
+  Acc a;
+  a.first(x0, y0);
+  a.add(x1, y1);
+  a.add(x2, y2);
+  return a.value();
+}
+__device__ __forceinline__ df2 dot4(df2 x0, df2 y0, df2 x1, df2 y1, df2 x2, df2 y2, df2 x3, df2 y3) {
+  Acc a;
+  a.first(x0, y0);
+  a.add(x1, y1);
+  a.add(x2, y2);
+  a.add(x3, y3);
+  return a.value();
+}
+__device__ __forceinline__ df2 pick(int c, df2 x0, df2 x1, df2 x2) { return c == 0 ? x0 : (c == 1 ? x1 : x2); }
 
 // a warp's shared memory: its faces' constants; for irregular patches also the
 // group's basis (float pairs) and the patch ids
@@ -152,9 +208,9 @@ __device__ __forceinline__ void split_faces(const DevBuf& b, const StepConst& sc
         for (int k = 1; k < 6; ++k) {
           if (RB[s][k] == 0) continue;
           if (s == 0)
-            a[k].first((float)RB[s][k], x[REG ? s : 0]);
+            a[k].first_int(RB[s][k], x[REG ? s : 0]);
           else
-            a[k].add((float)RB[s][k], x[REG ? s : 0]);
+            a[k].add_int(RB[s][k], x[REG ? s : 0]);
         }
       if (need_x) {
 #pragma unroll
@@ -175,44 +231,52 @@ __device__ __forceinline__ void split_faces(const DevBuf& b, const StepConst& sc
   __syncwarp();
   const df2* fc = w.face + f * kSplitStride;
   const df2 R00 = fc[SF_R00], R01 = fc[SF_R01], R10 = fc[SF_R10], R11 = fc[SF_R11];
-  const df2 du1 = R00 * G[1] + R10 * G[2], du2 = R01 * G[1] + R11 * G[2];
+  const df2 du1 = dot2(R00, G[1], R10, G[2]), du2 = dot2(R01, G[1], R11, G[2]);
   const df2 A1 = fc[SF_A1 + c], a1 = A1 + du1, a2 = fc[SF_A2 + c] + du2;
-  const df2 d1 = fc[SF_C11A] * G[3] + fc[SF_C11B] * G[4] + fc[SF_C11C] * G[5];
-  const df2 d2 = fc[SF_C22A] * G[3] + fc[SF_C22B] * G[4] + fc[SF_C22C] * G[5];
-  const df2 d3 = fc[SF_C12A] * G[3] + fc[SF_C12B] * G[4] + fc[SF_C12C] * G[5];
+  const df2 d1 = dot3(fc[SF_C11A], G[3], fc[SF_C11B], G[4], fc[SF_C11C], G[5]);
+  const df2 d2 = dot3(fc[SF_C22A], G[3], fc[SF_C22B], G[4], fc[SF_C22C], G[5]);
+  const df2 d3 = dot3(fc[SF_C12A], G[3], fc[SF_C12B], G[4], fc[SF_C12C], G[5]);
   // the sum of a value over the face's three lanes, in component order on each
   auto sum3 = [&](df2 v) { return (lane_of(v, base) + lane_of(v, base + 1)) + lane_of(v, base + 2); };
-  const df2 al0 = sum3((A1 + scale2(0.5f, du1)) * du1);
-  const df2 al1 = sum3((fc[SF_A2 + c] + scale2(0.5f, du2)) * du2);
-  const df2 al2 = sum3(A1 * du2 + du1 * a2);
+  // three such sums, one made by each lane and handed to the others
+  auto sum3x3 = [&](df2 v0, df2 v1, df2 v2, df2& s0, df2& s1, df2& s2) {
+    const df2 next = lane_of(pick(ck, v0, v1, v2), lj), prev = lane_of(pick(cj, v0, v1, v2), lk);
+    const df2 t = (pick(c, v0, v1, v2) + next) + prev;
+    s0 = lane_of(t, base); s1 = lane_of(t, base + 1); s2 = lane_of(t, base + 2);
+  };
+  df2 al0, al1, al2;
+  sum3x3((A1 + scale2(0.5f, du1)) * du1, (fc[SF_A2 + c] + scale2(0.5f, du2)) * du2, dot2(A1, du2, du1, a2), al0, al1,
+         al2);
   const df2 a2j = lane_of(a2, lj), a2k = lane_of(a2, lk);
   df2 Dn;
   {
     const df2 du1j = lane_of(du1, lj), du1k = lane_of(du1, lk), du2j = lane_of(du2, lj), du2k = lane_of(du2, lk);
-    Dn = (fc[SF_A1 + cj] * du2k - fc[SF_A1 + ck] * du2j) + (du1j * a2k - du1k * a2j);
+    Dn = dot4(fc[SF_A1 + cj], du2k, -fc[SF_A1 + ck], du2j, du1j, a2k, -du1k, a2j);
   }
   const df2 N0 = fc[SF_N + c], L0 = fc[SF_L0];
   const df2 dL2 = sum3((scale2(2.f, L0 * N0) + Dn) * Dn);  // |a1 x a2|^2 - L0^2
   const df2 jac = df_sqrt(L0 * L0 + dL2);
   const df2 invjac = df_recip(jac);
   const df2 s_n = -(dL2 * df_recip((L0 + jac) * jac));  // L0 / jac - 1
-  const df2 dn = Dn * invjac + N0 * s_n;
+  const df2 dn = dot2(Dn, invjac, N0, s_n);
   const df2 a3 = N0 + dn;
   const df2 D1 = fc[SF_D1 + c], D2 = fc[SF_D2 + c], D3 = fc[SF_D3 + c];
-  const df2 t0 = sum3(D1 * dn + d1 * a3), t1 = sum3(D2 * dn + d2 * a3), t2 = sum3(D3 * dn + d3 * a3);
+  df2 t0, t1, t2;
+  sum3x3(dot2(D1, dn, d1, a3), dot2(D2, dn, d2, a3), dot2(D3, dn, d3, a3), t0, t1, t2);
   const df2 h0 = fc[SF_B] + t0, h1 = fc[SF_B + 1] + t1, h2 = fc[SF_B + 2] + t2;
   // stress resultants times JxW: row c of H on lane c
   const df2 JxW = fc[SF_JXW];
-  df2 n0, n1, n2, m0, m1, m2, energy_n, energy_m;
+  df2 n0, n1, n2, m0, m1, m2, energy;  // energy: on lane 1 the membrane's, on lane 2 the bending's
   {
     const int q1 = c == 0 ? 1 : c + 2, q2 = c == 0 ? 2 : c + 3;
     const df2 Hc0 = fc[SF_H + c], Hc1 = fc[SF_H + q1], Hc2 = fc[SF_H + q2];
     const float on = (float)sc.internal_scale;  // 1, or 0 for the pressure-only force
-    const df2 n = (scale2(on, fc[SF_K]) * JxW) * (Hc0 * al0 + Hc1 * al1 + Hc2 * al2);
-    const df2 m = (scale2(-on, fc[SF_D]) * JxW) * (Hc0 * t0 + Hc1 * t1 + scale2(2.f, Hc2 * t2));
-    const df2 alc = c == 0 ? al0 : (c == 1 ? al1 : al2), tc = c == 0 ? t0 : (c == 1 ? t1 : scale2(2.f, t2));
-    energy_n = sum3(n * alc);
-    energy_m = -sum3(m * tc);
+    const df2 n = (scale2(on, fc[SF_K]) * JxW) * dot3(Hc0, al0, Hc1, al1, Hc2, al2);
+    const df2 m = (scale2(-on, fc[SF_D]) * JxW) * dot3(Hc0, t0, Hc1, t1, scale2(2.f, Hc2), t2);
+    const df2 en = n * pick(c, al0, al1, al2), em = -(m * pick(c, t0, t1, scale2(2.f, t2)));
+    const df2 en0 = lane_of(en, base), em0 = lane_of(em, base);
+    const df2 other = lane_of(c == 2 ? en : em, c == 1 ? base + 2 : base + 1);
+    energy = ((c == 1 ? en0 : em0) + (c == 1 ? en : em)) + other;
     n0 = lane_of(n, base); n1 = lane_of(n, base + 1); n2 = lane_of(n, base + 2);
     m0 = lane_of(m, base); m1 = lane_of(m, base + 1); m2 = lane_of(m, base + 2);
   }
@@ -231,25 +295,23 @@ __device__ __forceinline__ void split_faces(const DevBuf& b, const StepConst& sc
   if (valid) {
     // the measurements per unit area (area = jac / 2, and the metric's determinant is jac^2)
     const uint32_t e = __ldg(&b.perm[i]);
-    if (c == 0) {
-      b.area[e] = df_to_double(scale2(0.5f, jac));
-      b.etens[e] = df_to_double(energy_n * invjac);
-    } else if (c == 1) {
-      b.ebend[e] = df_to_double(energy_m * invjac);
-      b.kG[e] = df_to_double((h0 * h1 - h2 * h2) * invjac * invjac);
-    } else {
-      const df2 g0 = fc[SF_G] + scale2(2.f, al0), g1 = fc[SF_G + 1] + scale2(2.f, al1), g2 = fc[SF_G + 2] + al2;
-      b.kM[e] = df_to_double(scale2(0.5f, h0 * g1 + h1 * g0 - scale2(2.f, h2 * g2)) * invjac * invjac);
-    }
+    // (two values a lane: a value's conversion is FP64, 16 cycles of the SM's pipe)
+    const df2 g0 = fc[SF_G] + scale2(2.f, al0), g1 = fc[SF_G + 1] + scale2(2.f, al1), g2 = fc[SF_G + 2] + al2;
+    const df2 ei = energy * invjac;
+    double* to = c == 0 ? b.area : (c == 1 ? b.etens : b.ebend);
+    to[e] = df_to_double(c == 0 ? scale2(0.5f, jac) : ei);
+    // Gaussian curvature h0 h1 - h2 h2 on lane 1, mean (h0 g1 + h1 g0) / 2 - h2 g2 on lane 2
+    const df2 k = dot3(h0, c == 1 ? h1 : scale2(0.5f, g1), h1, c == 1 ? dfv(0.f) : scale2(0.5f, g0), -h2,
+                       c == 1 ? h2 : g2) * invjac * invjac;
+    if (c > 0) (c == 1 ? b.kG : b.kM)[e] = df_to_double(k);
   }
   df2 Y1, Y2;
   {
-    const df2 M = m0 * (D1 + d1) + m1 * (D2 + d2) + scale2(2.f, m2 * (D3 + d3));
-    const df2 sm = m0 * h0 + m1 * h1 + scale2(2.f, m2 * h2);
-    const df2 W = (M - sm * a3) * invjac;
+    const df2 sm = dot3(m0, h0, m1, h1, scale2(2.f, m2), h2);
+    const df2 W = dot4(m0, D1 + d1, m1, D2 + d2, scale2(2.f, m2), D3 + d3, -sm, a3) * invjac;
     const df2 Wj = lane_of(W, lj), Wk = lane_of(W, lk), a1j = lane_of(a1, lj), a1k = lane_of(a1, lk);
-    Y1 = n0 * a1 + n2 * a2 + (Wj * a2k - Wk * a2j);
-    Y2 = n1 * a2 + n2 * a1 + (a1j * Wk - a1k * Wj);
+    Y1 = dot4(n0, a1, n2, a2, Wj, a2k, -Wk, a2j);
+    Y2 = dot4(n1, a2, n2, a1, a1j, Wk, -a1k, Wj);
   }
   // pressure (ShellSystem.C:1509-1568), over the basis denominator on a regular patch
   constexpr double phi = REG ? 1.0 / 972.0 : 1.0;
@@ -275,11 +337,11 @@ __device__ __forceinline__ void split_faces(const DevBuf& b, const StepConst& sc
   const df2 y11 = -(m0 * a3), y22 = -(m1 * a3), y12 = -scale2(2.f, m2 * a3);
   df2 Z[6];
   Z[0] = -(JxW * pv);
-  Z[1] = fc[SF_R00] * Y1 + fc[SF_R01] * Y2;
-  Z[2] = fc[SF_R10] * Y1 + fc[SF_R11] * Y2;
-  Z[3] = fc[SF_C11A] * y11 + fc[SF_C22A] * y22 + fc[SF_C12A] * y12;
-  Z[4] = fc[SF_C11B] * y11 + fc[SF_C22B] * y22 + fc[SF_C12B] * y12;
-  Z[5] = fc[SF_C11C] * y11 + fc[SF_C22C] * y22 + fc[SF_C12C] * y12;
+  Z[1] = dot2(fc[SF_R00], Y1, fc[SF_R01], Y2);
+  Z[2] = dot2(fc[SF_R10], Y1, fc[SF_R11], Y2);
+  Z[3] = dot3(fc[SF_C11A], y11, fc[SF_C22A], y22, fc[SF_C12A], y12);
+  Z[4] = dot3(fc[SF_C11B], y11, fc[SF_C22B], y22, fc[SF_C12B], y12);
+  Z[5] = dot3(fc[SF_C11C], y11, fc[SF_C22C], y22, fc[SF_C12C], y12);
   auto put = [&](uint32_t at, df2 t) {
     reinterpret_cast<float2*>(b.qe)[3 * (size_t)at + c] = make_float2(t.h, t.l);
   };
@@ -287,10 +349,10 @@ __device__ __forceinline__ void split_faces(const DevBuf& b, const StepConst& sc
 #pragma unroll
     for (int s = 0; s < 12; ++s) {
       Acc a;
-      a.first((float)RB[s][0], Z[0]);
+      a.first_int(RB[s][0], Z[0]);
 #pragma unroll
       for (int k = 1; k < 6; ++k)
-        if (RB[s][k] != 0) a.add((float)RB[s][k], Z[k]);
+        if (RB[s][k] != 0) a.add_int(RB[s][k], Z[k]);
       if (valid) put(pos[REG ? s : 0], a.value());
     }
   } else {
