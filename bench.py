@@ -62,10 +62,10 @@ RUN_STEPS = 10000    # the length of the level-6 FP64 run
 # library kernels per step with self-contact: step start (k_begin_step, which also sets the
 # condition of the step's rebuild IF node), element kernel, contact force, gather/corrector
 # (which also predicts the next step), volume/measurement totals/end of step; plus, for each
-# rebuild, the body of the IF node: two linked-cell passes of 27 kernels (10 pipeline +
-# 3 x 3 scan + 8 contact CSR; the one not due returns at once) and the kernel between them
+# rebuild, the body of the IF node: two linked-cell passes of 23 kernels (10 pipeline +
+# 3 x 2 scan + 7 contact CSR; the one not due returns at once) and the kernel between them
 LAUNCHES_PER_STEP_CONTACT = 5
-LAUNCHES_PER_REBUILD = 55
+LAUNCHES_PER_REBUILD = 47
 # algorithmic bytes of one face-step of the FP64 path: vertex state u, v, a read and written
 # plus M^-1 and C (96 B per face), per-face constants (R, reference metric, forms, stiffness,
 # JxW: 264 B), connectivity and CSR (96 B); intermediate force shares are not counted

@@ -1262,7 +1262,7 @@ shl_status begin_eval(shl_ctx* c, double pressure, bool allow_rebuild, ListDue& 
   return SHL_OK;
 }
 
-// The 25 kernels of list work that is not due would each return at once, but
+// The kernels of list work that is not due would each return at once, but
 // launching them took 110 of the 252 us of a call (27,380 faces; now 144 us).
 shl_status eval_into(shl_ctx* c, double* d_f, double* d_a, const ListDue& due) {
   const DevBuf& b = c->b;

@@ -23,7 +23,8 @@
 //   scan, k_rb_scatter_new  accepted pairs grouped by eid1 (counting sort)
 //   scan           per-face pair counts -> segment offsets
 //   k_rb_assemble  kept old pairs + new pairs of each face, merged in e2 order
-//   k_rb_copyback  scratch list -> list
+//   k_rb_copyback  scratch list -> list; its last block ends the pass
+//   k_csr_*, scan  each node's (pair, role) entries, sorted
 //
 // The resulting list equals, as a set, the reference's list at the same state
 // (the reference's cell-membership test is reproduced with the same rounded
@@ -1302,15 +1303,10 @@ __global__ void k_rb_copyback(DevBuf b, StepConst sc) {
       for (int c = 0; c < 4; ++c) b.pvw[0][4 * (size_t)j + c] = b.pvw[1][4 * (size_t)j + c];
   }
   for (uint32_t f = blockIdx.x * blockDim.x + threadIdx.x; f <= sc.F; f += stride) b.pair_ptr[0][f] = b.pair_ptr[1][f];
-}
-
-// flag flip after the copy-back (after all blocks are done); a batch also
-// clears its shells' flags
-__global__ void k_rb_finish(DevBuf b, StepConst sc) {
-  Ctl* ctl = b.ctl;
-  if (rb_off(ctl)) return;
+  // the last block ends the pass (every block has read its flag); a batch also
+  // clears its shells' flags
+  if (!last_block_rb(&ctl->cnt[10])) return;
   for (uint32_t s = threadIdx.x; s < sc.n_cs; s += blockDim.x) b.shc[s].rebuild = 0;
-  __syncthreads();
   if (threadIdx.x != 0) return;
   ctl->n_pairs = ctl->n_next;
   ctl->rebuild = 0;
@@ -1412,6 +1408,7 @@ __global__ void __launch_bounds__(kCsrSortBigBlock) k_csr_sort_big(DevBuf b, Ste
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) b.csr_ent[k0 + i] = big[i];
     __syncthreads();
   }
+  if (last_block_rb(&ctl->cnt[11]) && threadIdx.x == 0) ctl->csr_dirty = 0;
 }
 
 // Bitonic sort of n <= 32 E entries by one warp, in registers: element
@@ -1487,11 +1484,6 @@ __global__ void __launch_bounds__(32 * kCsrSortWarps) k_csr_sort(DevBuf b, StepC
   }
 }
 
-__global__ void k_csr_finish(DevBuf b) {
-  if (csr_off(b.ctl)) return;
-  b.ctl->csr_dirty = 0;
-}
-
 inline uint32_t nblk(uint32_t n, uint32_t bs = kBlock) { return n == 0 ? 1 : (n + bs - 1) / bs; }
 
 }  // namespace
@@ -1550,7 +1542,6 @@ void launch_contact_csr(const DevBuf& b, const StepConst& sc, cudaStream_t s) {
     k_csr_sort<<<g ? g : 1, 32 * kCsrSortWarps, 0, s>>>(b, sc);
     k_csr_sort_big<<<152, kCsrSortBigBlock, kCsrSortBigCap * 4, s>>>(b, sc);
   }
-  k_csr_finish<<<1, 1, 0, s>>>(b);
 }
 
 void launch_rebuild(const DevBuf& b, const StepConst& sc, cudaStream_t s) {
@@ -1608,7 +1599,6 @@ void launch_rebuild(const DevBuf& b, const StepConst& sc, cudaStream_t s) {
     if (g > 8 * 152) g = 8 * 152;
     k_rb_copyback<<<g, kBlock, 0, s>>>(b, sc);
   }
-  k_rb_finish<<<1, sc.n_cs ? kBlock : 32, 0, s>>>(b, sc);
   launch_contact_csr(b, sc, s);
 }
 
