@@ -2218,9 +2218,13 @@ __global__ void __launch_bounds__(kBlock) k_gather_correct(DevBuf b, StepConst s
 // contact (its per-node scalar work would be repeated on three lanes) and for the
 // adaptive attempt's norms.
 constexpr int kNodeLanes = 3, kNodesPerWarp = 10, kGatherChunk = kNodesPerWarp * (kBlock / 32);
-constexpr uint32_t kGatherBlocks = 152 * 6;  // a block takes every gridDim.x-th chunk of 80 nodes
+// A block takes every gridDim.x-th chunk of 80 nodes; the grid is what the SMs
+// hold at once (with 912 blocks on 608 places, the second round half filled: 82 k
+// nodes 153 us a relaxation step, now 140; level 7 FP32 168 -> 156 us a step; five
+// or six blocks an SM with fewer registers are between).
+constexpr uint32_t kGatherPerSm = 4, kGatherBlocks = 152 * kGatherPerSm;
 
-__global__ void __launch_bounds__(kBlock) k_gather_lanes(DevBuf b, StepConst sc, int mode, double* f_out, double* a_out,
+__global__ void __launch_bounds__(kBlock, kGatherPerSm) k_gather_lanes(DevBuf b, StepConst sc, int mode, double* f_out, double* a_out,
                                                          RebuildCond rc) {
   // modes as in k_gather_correct (not 2)
   Ctl* ctl = b.ctl;
@@ -2247,6 +2251,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_lanes(DevBuf b, StepConst sc,
                  s_m = corr ? b.M[k] : 0.0;
     double f = 0.0;
     const uint32_t nn = on ? n : n0;
+    const uint32_t g0 = b.gather_ptr[nn], g1 = b.gather_ptr[nn + 1];
     if (sc.contact) {
       const uint32_t k1 = b.csr_ptr[nn + 1];
 #pragma unroll 8
@@ -2258,7 +2263,6 @@ __global__ void __launch_bounds__(kBlock) k_gather_lanes(DevBuf b, StepConst sc,
         f = fma(role < 3 ? -w : w, pf[c], f);
       }
     }
-    const uint32_t g0 = b.gather_ptr[nn], g1 = b.gather_ptr[nn + 1];
     if (sc.fp32) {
       float s0 = 0.f;
       const float* q = b.qe32 + c;

@@ -2,7 +2,7 @@
 by the mesh.
 
 A batch of nine level-5 shells has more nodes than one round of the gather's and
-of the contact sort's grids (72,960 and 77,824), more cells than one round of the
+of the contact sort's grids (48,640 and 77,824), more cells than one round of the
 scan's (2.5 million) and face counts that leave a partly filled warp: it must
 equal a shell run alone, which needs one round, bit for bit.  The cavity's node
 blocks are 32, 64, 128 or 256 threads: forces within the 1e-12 of the other
