@@ -74,20 +74,21 @@ STEP_BYTES_PER_FACE = 456
 # arithmetic in element_force<12>, fused multiply-add = 2)
 ELEM_FLOPS_PER_FACE = 1372
 # DRAM bytes (read + write) of one launch of the tuned element kernel (the
-# one-round double-float shape, 544 threads per SM) on the level-6 shell, from
-# one ncu --set full capture with caches flushed (46.3 MB read, 15.9 MB written)
-ELEM_TRAFFIC_LEVEL6 = 62.2e6
+# component-split kernel, 64 x 12) on the level-6 shell, from one ncu capture with
+# caches flushed (44.6 MB read, 0.7 MB written: the shares stay in L2)
+ELEM_TRAFFIC_LEVEL6 = 45.3e6
 # FP32 element path (the ensemble): about 300 algorithmic bytes per face-step with
 # FP32 per-face constants; DRAM bytes of one launch on the 256-shell ensemble and its
-# FP32-pipe utilisation, from one ncu --set full capture (673.4 MB read, 427.0 MB
-# written: the force shares do not fit in L2 at this size)
+# (671.3 MB read, 407.9 MB written: the force shares do not fit in L2 at this size;
+# one ncu capture) and the FP32-pipe utilisation of the same arithmetic before its
+# constants came as records (a lower bound now)
 ENS_BYTES_PER_FACE = 300
-ENS_ELEM_TRAFFIC = 1100.4e6
+ENS_ELEM_TRAFFIC = 1079.2e6
 ENS_ELEM_FP32_PIPE = 0.129
 # warp instructions of one element-kernel launch on the level-6 shell (ncu
 # smsp__inst_executed.sum of the same capture) and the issue peak: 4 schedulers
 # per SM, one warp instruction per cycle each
-ELEM_WARP_INST_LEVEL6 = 30.7e6
+ELEM_WARP_INST_LEVEL6 = 22.95e6
 ISSUE_PER_SM_PER_CYCLE = 4
 
 
