@@ -246,7 +246,7 @@ struct DevBuf {
   uint32_t* tri;      // 3F original order
   uint32_t *perm;     // internal -> original
   double *area, *kG, *kM, *etens, *ebend;  // original order
-  double *area_odd, *kG_odd, *kM_odd, *etens_odd, *ebend_odd;  // the same fields of every other pipelined step
+  double *area_odd, *kG_odd, *kM_odd, *etens_odd, *ebend_odd;  // second set: every other pipelined step
   double* partial;    // per-block partial sums
   double* partial_v;  // those of the measurement (k_volume_end), which runs beside other kernels
   uint32_t *close_ptr, *close_list;
@@ -362,8 +362,10 @@ void launch_contact_force(const DevBuf& b, const StepConst& sc, int cur, cudaStr
 void launch_gather_correct(const DevBuf& b, const StepConst& sc, int mode, bool correct, double* f_out,
                            double* a_out, cudaStream_t s, RebuildCond rc = {0, 0});
 // the measurement totals and the volume (kVolTotals), with the end of the step
-// (kVolEndStep), or with the report's sums of a pipelined step (kVolMeasure)
-enum : int { kVolTotals = 0, kVolEndStep = 1, kVolMeasure = 2 };
+// (kVolEndStep), or with the report's sums of a pipelined step (kVolMeasure; with
+// its per-face fields in the second set, kVolMeasureOdd: the buffer table has the
+// two sets exchanged, and a run that stopped gets its fields in the first)
+enum : int { kVolTotals = 0, kVolEndStep = 1, kVolMeasure = 2, kVolMeasureOdd = 3 };
 void launch_volume_end_step(const DevBuf& b, const StepConst& sc, int mode, cudaStream_t s);
 void launch_positions(const DevBuf& b, const StepConst& sc, cudaStream_t s);
 // u, v, a between the context and mapped page-locked host memory (device pointers of it)

@@ -2445,7 +2445,7 @@ __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, i
   Ctl* ctl = b.ctl;
   const bool end_step = mode == kVolEndStep;
   // a pipelined step was ended by its corrector, which may have stopped the run
-  if (mode == kVolMeasure ? ctl->measure == 0 : inactive(ctl)) return;
+  if (mode >= kVolMeasure ? ctl->measure == 0 : inactive(ctl)) return;
   if (end_step && sc.adapt_every && !ctl->accept) {
     // a repeated attempt ends no step; only a step size below the machine
     // precision (SHL_SMALL_TIMESTEP) ends the run (ShellSystem.C:1110-1117)
@@ -2467,6 +2467,14 @@ __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, i
   double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   if (f < sc.F) {
     face_totals(b, f, v);
+    // a run that stopped with this step reads its fields from the first set
+    if (mode == kVolMeasureOdd && inactive(ctl)) {
+      b.area_odd[f] = b.area[f];
+      b.kG_odd[f] = b.kG[f];
+      b.kM_odd[f] = b.kM[f];
+      b.etens_odd[f] = b.etens[f];
+      b.ebend_odd[f] = b.ebend[f];
+    }
     const double* q0 = b.p + 3 * (size_t)b.tri[3 * (size_t)f];
     const double* q1 = b.p + 3 * (size_t)b.tri[3 * (size_t)f + 1];
     const double* q2 = b.p + 3 * (size_t)b.tri[3 * (size_t)f + 2];
