@@ -55,9 +55,11 @@ __device__ __forceinline__ void pair_compute_block(bool active, const double* co
     const double* const q2[3] = {q[1][0], q[1][1], q[1][2]};
     mask = shl_pair_mask(q1, q2);
   }
-  // the best test so far: its d2 as bits (d2 is a sum of squares or NaN, whose
-  // bits compare as integers the way the doubles do; no NaN is below DBL_MAX)
-  long long best = __double_as_longlong(SHL_DBL_MAX);
+  // the best test so far: its d2 as bits.  d2 is a sum of squares, whose bits
+  // compare as unsigned integers the way the doubles do, or NaN, whose bits with
+  // either sign are above DBL_MAX's (a face without area gives 0/0, and the
+  // device's NaN has its sign set: as a signed integer it would be the smallest)
+  unsigned long long best = (unsigned long long)__double_as_longlong(SHL_DBL_MAX);
   int best_k = -1;
   double dc[3] = {0.0, 0.0, 0.0}, par[2] = {0.0, 0.0};
 #pragma unroll 1
@@ -121,7 +123,7 @@ __device__ __forceinline__ void pair_compute_block(bool active, const double* co
       __syncthreads();
       for (; at < end && at < base + kPairBlock; ++at) {
         const uint32_t r = at - base;
-        const long long d2 = __double_as_longlong(w.res[0][r]);
+        const unsigned long long d2 = (unsigned long long)__double_as_longlong(w.res[0][r]);
         if (d2 < best) {
           best = d2;
           best_k = (int)(w.item[at] & 15u) + 9 * vertex;
@@ -133,7 +135,7 @@ __device__ __forceinline__ void pair_compute_block(bool active, const double* co
     }
   }
   shl_pair_none(g);
-  const double d2 = __longlong_as_double(best);
+  const double d2 = __longlong_as_double((long long)best);
   if (best_k >= 9)
     shl_pair_take_vertex((best_k - 9) / 3, (best_k - 9) % 3, d2, dc, par, g);
   else if (best_k >= 0)

@@ -19,9 +19,11 @@
  *    of its coefficients: for nearly parallel edges the parameter error grows,
  *    but the quadratic flattens in proportion, and the end that a clamped
  *    parameter takes follows the sign of the numerator, not of the vanishing
- *    determinant.  Largest difference from FP64 in 6e8 edge pairs (layers,
- *    slivers, parallel, touching, needle edges): 20 eps; the bound allows
- *    SHL_PRUNE_E = 128 eps.
+ *    determinant.  Largest difference from FP64 (layers, slivers, parallel,
+ *    touching, needle edges): 20 eps in 6e8 edge pairs of a host build (no
+ *    contraction, true division); 13 eps in the 1e7 edge pairs that the GPU test
+ *    of the block search sends through the device build (contraction, fast
+ *    division).  The bound allows SHL_PRUNE_E = 128 eps.
  *  - Vertex-face.  Projection clearly outside: the minimum over the face's
  *    three edges (same bound).  Otherwise the plane's distance, less its
  *    rounding (SHL_PRUNE_P eps / sin of the corner angle).  A face with a
