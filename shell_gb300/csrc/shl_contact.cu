@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "shl_cells.h"
 #include "shl_geom.h"
 #include "shl_internal.cuh"
 #include "shl_pairs.cuh"
@@ -380,13 +381,8 @@ constexpr uint32_t kWideFaces = 8192;
 // the cells lo..hi of a face, G lanes at a time: calls at(cell)
 template <int G, class Fn>
 __device__ __forceinline__ void walk_cells(const GridView& g, const int* lo, const int* hi, uint32_t sub, Fn at) {
-  const uint32_t ny = g.ny, nz = g.nz;
-  const uint32_t cy = (uint32_t)(hi[1] - lo[1] + 1), cz = (uint32_t)(hi[2] - lo[2] + 1);
-  const uint32_t total = (uint32_t)(hi[0] - lo[0] + 1) * cy * cz;
-  for (uint32_t q = sub; q < total; q += G) {
-    const uint32_t z = q % cz, y = q / cz % cy, x = q / (cz * cy);
-    at(g.base + ((uint32_t)lo[0] + x) * ny * nz + ((uint32_t)lo[1] + y) * nz + (uint32_t)lo[2] + z);
-  }
+  const uint32_t total = shl_cells_covered(lo, hi);
+  for (uint32_t q = sub; q < total; q += G) at(g.base + shl_cells_at(q, lo, hi, g.ny, g.nz));
 }
 
 // cell ranges (ShellSystem.C:1982-1983) and histogram of the faces (G = 1 or a
