@@ -137,6 +137,7 @@ shl_status dev_alloc(shl_ctx* c, T** p, size_t n) {
   cudaError_t e = cudaMalloc(&q, bytes);
   if (e != cudaSuccess) {
     g_err = "cudaMalloc(" + std::to_string(bytes) + "): " + cudaGetErrorString(e);
+    cudaGetLastError();  // reported here: the next launch check must not find it again
     return SHL_ERR_OOM;
   }
   // zero on the context stream: the stream is non-blocking, so a default-stream
@@ -1913,24 +1914,27 @@ shl_status shl_residual(shl_ctx* c, double pressure, int flags, double* rel, dou
     g_err = "SHL_RESIDUAL_CONTACT needs self-contact without friction";
     return SHL_ERR_ARG;
   }
+  // each buffer by its own check: an earlier call may have found memory for the first ones only
+  if (!c->d_norms) SHL_TRY(dev_alloc(c, &c->d_norms, 2 * (size_t)ns));
   if (!c->d_node_off) {
     SHL_TRY(dev_alloc(c, &c->d_node_off, ns + 1));
-    SHL_TRY(dev_alloc(c, &c->d_norms, 2 * (size_t)ns));
     SHL_CUDA_TRY(cudaMemcpyAsync(c->d_node_off, c->node_off.data(), (ns + 1) * sizeof(uint32_t),
                                  cudaMemcpyHostToDevice, c->stream));
   }
-  if (fp64 && ctx32 && !c->qe64) SHL_TRY(dev_alloc(c, &c->qe64, 3 * (size_t)c->S.n_slots_total));
-  if (fp64 && ctx32 && !c->b.face_df) {  // the double-float FP64 path's constants
-    SHL_TRY(dev_alloc(c, &c->b.face_df, 2 * c->S.split.size()));
-    SHL_TRY(upload_split(c));
-    if (c->sc.smooth) {
+  if (fp64 && ctx32) {  // the double-float FP64 path's shares and constants
+    if (!c->qe64) SHL_TRY(dev_alloc(c, &c->qe64, 3 * (size_t)c->S.n_slots_total));
+    if (!c->b.face_df) {
+      SHL_TRY(dev_alloc(c, &c->b.face_df, 2 * c->S.split.size()));
+      SHL_TRY(upload_split(c));
+    }
+    if (c->sc.smooth && !c->b.face_soa) {
       SHL_TRY(dev_alloc(c, &c->b.face_soa, c->S.face_soa.size()));
       SHL_TRY(upload(c, c->b.face_soa, c->S.face_soa.data(), c->S.face_soa.size()));
     }
   }
+  if (correct && !c->f32) SHL_TRY(dev_alloc(c, &c->f32, nd));
   if (correct && !c->b.fcorr) {
     SHL_TRY(dev_alloc(c, &c->b.fcorr, nd));
-    SHL_TRY(dev_alloc(c, &c->f32, nd));
     // the step graphs hold the buffer table by value: capture them again with the correction
     if (c->graph) cudaGraphExecDestroy(c->graph);
     if (c->graph1) cudaGraphExecDestroy(c->graph1);
