@@ -27,12 +27,16 @@ namespace {
 thread_local std::string g_err;
 constexpr uint32_t kGraphSteps = 16;
 constexpr uint32_t kTableCap = 1u << 16;
-// Subdivision levels times irregular faces whose children's power forms are made
-// before each SMOOTH search: all 34 levels of the 60 faces around a sphere's
-// twelve irregular vertices, about 10 us of FP64 work and 2 MB; meshes with more
-// irregular faces keep their first levels (level 1 is three quarters of a patch's
-// parameter area, level 2 three quarters of the rest, and so on) or none.
-constexpr uint32_t kIrregularLevels = 2048;
+// Subdivision levels of the irregular faces whose children's power forms are made
+// before each SMOOTH search: all 34 for up to kIrregularLevels / 34 faces (the 60
+// around a sphere's twelve irregular vertices: about 10 us of FP64 work and 2 MB),
+// beyond that as many as this number gives each face, and no fewer than
+// kIrregularMin: the first levels and the last (stored_slot), 8.6 KB a face.  A
+// search beyond them makes the form itself, over and over.  Four steps of a folded
+// irregular mesh of 5,120 faces with 2, 4 and 8 levels: 328, 243 and 226 ms (without
+// any 476); of 200 folded level-2 spheres 47, 42 and 35 ms (117); the forms
+// themselves take 0.2 and 0.5 ms of a step.
+constexpr uint32_t kIrregularLevels = 2048, kIrregularMin = 8;
 
 #define SHL_CUDA_TRY(expr)                                                 \
   do {                                                                     \
@@ -838,7 +842,7 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
       irr_first = S.groups[0].count;
       const uint32_t n_irr = F - irr_first;
       if (n_irr) {
-        irr_levels = (int32_t)std::min<uint32_t>(SHL_SMOOTH_LEVELS, kIrregularLevels / n_irr);
+        irr_levels = (int32_t)std::min<uint32_t>(SHL_SMOOTH_LEVELS, std::max(kIrregularLevels / n_irr, kIrregularMin));
         ALLOC(b.icoef, (size_t)n_irr * irr_levels * 3 * SHL_LIMIT_NCOEF);
       }
       ALLOC(b.inv_perm, F); ALLOC(b.fsm, F);

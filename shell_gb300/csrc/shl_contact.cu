@@ -812,7 +812,7 @@ __global__ void __launch_bounds__(kBlock) k_limit_coeffs(DevBuf b, StepConst sc,
     if (t < n_irr) {
       const int c = (int)(t % 3u), k = (int)(t / 3u % 3u);
       const uint32_t q = t / 9u;
-      const int n = 1 + (int)(q % (uint32_t)sc.irr_levels);
+      const int slot = (int)(q % (uint32_t)sc.irr_levels), n = slot == sc.irr_levels - 1 ? SHL_SMOOTH_LEVELS : 1 + slot;
       shl_limit_patch lp;
       smooth_patch(b, sc, b.perm[sc.irr_first + q / (uint32_t)sc.irr_levels], lp);
       SHL_TABLE signed char BC[12][15] = SHL_BOX_COEFFS;
@@ -844,25 +844,33 @@ __global__ void __launch_bounds__(kBlock) k_limit_coeffs(DevBuf b, StepConst sc,
   }
 }
 
+// the place of subdivision level n among a patch's stored levels, the first
+// levels - 1 and the last one (the patch's corner, where many a search ends), or -1
+__device__ __forceinline__ int stored_slot(int n, int levels) {
+  return n == SHL_SMOOTH_LEVELS ? levels - 1 : (n < levels ? n - 1 : -1);
+}
+
 // a patch's limit surface at (v, w) from the stored power forms; deep: also the
-// levels of an irregular patch beyond them
+// levels of an irregular patch beyond them (the form is made here; the lanes of
+// a batch evaluate theirs together)
 template <int ORDER, bool DEEP>
 __device__ __noinline__ void limit_at(const DevBuf& b, const StepConst& sc, uint32_t e, double v, double w, double out[6][3]) {
   double j1 = 1.0;
   const double* coef = b.lcoef + SHL_LIMIT_NCOEF * (size_t)e;
+  double P[15][3];
   if ((b.fsm[e] & 0xff) != 6) {
     int n, k;
     shl_limit_child(&v, &w, &n, &k, &j1);
-    if (DEEP && n > sc.irr_levels) {
+    const int slot = stored_slot(n, sc.irr_levels);
+    if (DEEP && slot < 0) {
       shl_limit_patch lp;
       smooth_patch(b, sc, e, lp);
-      double P[15][3];
       shl_limit_coeffs_child(&lp, n, k, P);
-      shl_limit_poly(P, v, w, ORDER, j1, out);
-      return;
+      coef = &P[0][0];
+    } else {
+      coef = b.icoef +
+             SHL_LIMIT_NCOEF * ((size_t)((b.inv_perm[e] - sc.irr_first) * (uint32_t)sc.irr_levels + (uint32_t)slot) * 3 + (size_t)k);
     }
-    coef = b.icoef +
-           SHL_LIMIT_NCOEF * ((size_t)((b.inv_perm[e] - sc.irr_first) * (uint32_t)sc.irr_levels + (uint32_t)(n - 1)) * 3 + (size_t)k);
   }
   shl_limit_poly(reinterpret_cast<const double(*)[3]>(coef), v, w, ORDER, j1, out);
 }
@@ -874,9 +882,12 @@ __device__ __noinline__ void limit_at(const DevBuf& b, const StepConst& sc, uint
 // lanes of a warp sit in different phases, and every trip pays for both with a
 // third of the lanes busy in each.  Here a warp owns kSearchPool searches, kept
 // in shared memory as resumable states (shl_smooth_state), and per trip runs up
-// to 32 of them that are in the same phase; searches with an irregular patch
-// that may have to subdivide beyond the stored children are a class of their own.  With more searches
-// than lanes there is nearly always a full batch of one class.  A finished
+// to 32 of them that are in the same phase.  A search whose next point lies in an
+// irregular patch beyond the stored children makes a power form for it, which
+// costs more than the rest of a trip; those are classes of their own, again one
+// per phase (as one class, for every search with an irregular patch, they made
+// batches and irregular meshes up to 1.9 times slower than a search per lane).
+// With more searches than lanes there is nearly always a full batch of one class.  A finished
 // search's slot is refilled from a queue shared by the grid (ctl->cnt[7]; the
 // last warp to leave resets it).  A search's result does not depend on the lane
 // or the order that runs it.  Folded level-5 shell, 1.4 M candidates at 5.9
@@ -894,13 +905,14 @@ __device__ __noinline__ void limit_at(const DevBuf& b, const StepConst& sc, uint
 //   k_contact_force.
 constexpr int kSearchBlock = 128;
 constexpr int kSearchPool = 64;  // searches per warp (a multiple of 32)
-enum : uint8_t { kSearchEmpty = 0, kSearchNewton = 1, kSearchTrial = 2, kSearchDeep = 3 };
+enum : uint8_t { kSearchEmpty = 0, kSearchNewton = 1, kSearchTrial = 2, kSearchDeep = 2 };  // + kSearchDeep: 3, 4
+constexpr int kSearchClasses = 5;
 struct SearchPool {
   double x[4][kSearchPool], xt[4][kSearchPool], d[4][kSearchPool], p1[3][kSearchPool], p2[3][kSearchPool];
   double f[kSearchPool], alpha[kSearchPool], gd[kSearchPool], dn[kSearchPool];
   uint32_t j[kSearchPool], e1[kSearchPool], e2[kSearchPool];
-  uint8_t cls[kSearchPool], trial[kSearchPool], it[kSearchPool], ls[kSearchPool], shifted[kSearchPool],
-      after_accept[kSearchPool];
+  uint8_t cls[kSearchPool], it[kSearchPool], ls[kSearchPool], shifted[kSearchPool], after_accept[kSearchPool];
+  uint8_t irregular[kSearchPool];  // bit 0 / 1: element 1 / 2 has an irregular patch
   uint8_t batch[32];
 };
 
@@ -983,19 +995,37 @@ __device__ __forceinline__ void search_trip(const DevBuf& b, const StepConst& sc
       }
     }
   }
-  const bool trial = st.phase == SHL_SMOOTH_EVAL_TRIAL;
-  w.trial[s] = trial ? 1 : 0;
-  if (!DEEP) w.cls[s] = trial ? kSearchTrial : kSearchNewton;
+  w.cls[s] = st.phase == SHL_SMOOTH_EVAL_TRIAL ? kSearchTrial : kSearchNewton;
 }
 
-// trips of the deep class, out of line: they are rare, and their copy of the
-// evaluation would crowd the others out of the instruction cache
-template <bool REBUILD>
-__device__ __noinline__ void search_trip_deep(const DevBuf& b, const StepConst& sc, Ctl* ctl, SearchPool& w, uint32_t s) {
-  search_trip<REBUILD, true>(b, sc, ctl, w, s, w.trial[s] ? SHL_SMOOTH_EVAL_TRIAL : SHL_SMOOTH_EVAL_FGH);
+// a search of the shallow classes moves to the deep ones if its next point lies in
+// an irregular patch beyond the stored levels
+__device__ __noinline__ void deepen(SearchPool& w, uint32_t s, int levels) {
+  const unsigned irr = w.irregular[s], cls = w.cls[s];
+  if (irr == 0 || cls == kSearchEmpty) return;
+  const double(*pt)[kSearchPool] = cls == kSearchTrial ? w.xt : w.x;
+  for (int k = 0; k < 2; ++k) {
+    if (!(irr >> k & 1u)) continue;
+    double v = pt[2 * k][s], x = pt[2 * k + 1][s];
+    if (stored_slot(shl_rescale_irregular(&v, &x), levels) < 0) {
+      w.cls[s] = (uint8_t)(cls + kSearchDeep);
+      return;
+    }
+  }
 }
 
+// trips of the deep classes, out of line: they are rare on most meshes, and their
+// copy of the evaluation would crowd the others out of the instruction cache
 template <bool REBUILD>
+__device__ __noinline__ void search_trip_deep(const DevBuf& b, const StepConst& sc, Ctl* ctl, SearchPool& w, uint32_t s,
+                                              int phase) {
+  search_trip<REBUILD, true>(b, sc, ctl, w, s, phase);
+}
+
+// DEEP: not every level of every irregular patch is stored (sc.irr_levels).  With
+// all of them, the deep classes and their calls are left out of the kernel, which
+// as a branch of it cost a sphere's searches 2 to 4 %.
+template <bool REBUILD, bool DEEP>
 __global__ void __launch_bounds__(kSearchBlock, 2) k_smooth_search(DevBuf b, StepConst sc) {
   Ctl* ctl = b.ctl;
   uint32_t* queue = &ctl->cnt[7];
@@ -1014,12 +1044,13 @@ __global__ void __launch_bounds__(kSearchBlock, 2) k_smooth_search(DevBuf b, Ste
   while (n > 0) {
     // slots of each class
     uint8_t cl[R];
-    unsigned count[4] = {0, 0, 0, 0};
+    constexpr int kClasses = DEEP ? kSearchClasses : kSearchTrial + 1;
+    unsigned count[kClasses] = {};
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       cl[r] = w.cls[32 * r + lane];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) count[k] += __popc(__ballot_sync(0xffffffffu, cl[r] == k));
+      for (int k = 0; k < kClasses; ++k) count[k] += __popc(__ballot_sync(0xffffffffu, cl[r] == k));
     }
     if (more && count[kSearchEmpty] >= 16) {
       // refill the empty slots
@@ -1053,17 +1084,20 @@ __global__ void __launch_bounds__(kSearchBlock, 2) k_smooth_search(DevBuf b, Ste
         for (int k = 0; k < 4; ++k) w.x[k][s] = st.x[k];
         w.it[s] = 0;
         w.after_accept[s] = 0;
-        w.trial[s] = 0;
-        const bool kept = sc.irr_levels == SHL_SMOOTH_LEVELS || ((b.fsm[e1] & 0xff) == 6 && (b.fsm[e2] & 0xff) == 6);
-        w.cls[s] = kept ? kSearchNewton : kSearchDeep;
+        w.cls[s] = kSearchNewton;
+        if (DEEP) {
+          w.irregular[s] = (uint8_t)(((b.fsm[e1] & 0xff) != 6 ? 1u : 0u) | ((b.fsm[e2] & 0xff) != 6 ? 2u : 0u));
+          deepen(w, s, sc.irr_levels);
+        }
       }
       __syncwarp();
       continue;
     }
     // the largest class runs a batch
     int pick = kSearchNewton;
-    if (count[kSearchTrial] > count[pick]) pick = kSearchTrial;
-    if (count[kSearchDeep] > count[pick]) pick = kSearchDeep;
+#pragma unroll
+    for (int k = kSearchTrial; k < kClasses; ++k)
+      if (count[k] > count[pick]) pick = k;
     if (count[pick] == 0) break;  // no search left (the queue is empty: an empty pool would have been refilled)
     uint32_t pos = 0;
 #pragma unroll
@@ -1080,8 +1114,10 @@ __global__ void __launch_bounds__(kSearchBlock, 2) k_smooth_search(DevBuf b, Ste
         search_trip<REBUILD, false>(b, sc, ctl, w, s, SHL_SMOOTH_EVAL_FGH);
       else if (pick == kSearchTrial)
         search_trip<REBUILD, false>(b, sc, ctl, w, s, SHL_SMOOTH_EVAL_TRIAL);
-      else
-        search_trip_deep<REBUILD>(b, sc, ctl, w, s);
+      else if (DEEP)
+        search_trip_deep<REBUILD>(b, sc, ctl, w, s,
+                                  pick == kSearchTrial + kSearchDeep ? SHL_SMOOTH_EVAL_TRIAL : SHL_SMOOTH_EVAL_FGH);
+      if (DEEP) deepen(w, s, sc.irr_levels);
     }
     __syncwarp();
   }
@@ -1484,30 +1520,36 @@ inline uint32_t nblk(uint32_t n, uint32_t bs = kBlock) { return n == 0 ? 1 : (n 
 
 }  // namespace
 
+constexpr size_t kSearchSmem = sizeof(SearchPool) * (kSearchBlock / 32);
+
 // a grid that the SMs hold at once (the queue hands out the pairs)
-template <bool REBUILD>
+template <bool REBUILD, bool DEEP>
 static uint32_t search_grid() {
   static const uint32_t g = [] {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_smooth_search<REBUILD>, kSearchBlock,
-                                                  sizeof(SearchPool) * (kSearchBlock / 32));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_smooth_search<REBUILD, DEEP>, kSearchBlock, kSearchSmem);
     return (uint32_t)(sms > 0 ? sms : 152) * (uint32_t)(per_sm > 0 ? per_sm : 1);
   }();
   return g;
+}
+
+template <bool REBUILD, bool DEEP>
+static void launch_search(const DevBuf& b, const StepConst& sc, cudaStream_t s) {
+  k_smooth_search<REBUILD, DEEP><<<search_grid<REBUILD, DEEP>(), kSearchBlock, kSearchSmem, s>>>(b, sc);
 }
 
 void launch_smooth_search(const DevBuf& b, const StepConst& sc, bool rebuild, cudaStream_t s) {
   uint32_t g = nblk(sc.F);
   if (g > 8 * 152) g = 8 * 152;
   if (sc.F > sc.irr_first && g < 152) g = 152;  // the irregular children, hundreds per face
-  constexpr size_t smem = sizeof(SearchPool) * (kSearchBlock / 32);
   k_limit_coeffs<<<g, kBlock, 0, s>>>(b, sc, rebuild);
+  const bool deep = sc.irr_levels < SHL_SMOOTH_LEVELS;
   if (rebuild)
-    k_smooth_search<true><<<search_grid<true>(), kSearchBlock, smem, s>>>(b, sc);
+    deep ? launch_search<true, true>(b, sc, s) : launch_search<true, false>(b, sc, s);
   else
-    k_smooth_search<false><<<search_grid<false>(), kSearchBlock, smem, s>>>(b, sc);
+    deep ? launch_search<false, true>(b, sc, s) : launch_search<false, false>(b, sc, s);
 }
 
 // kernels that take more than the default 48 KB of shared memory; called once
@@ -1518,9 +1560,10 @@ cudaError_t init_contact_kernels() {
   };
   cudaError_t e = set((const void*)k_rb_narrow, sizeof(PairWork));
   if (e == cudaSuccess) e = set((const void*)k_csr_sort_big, kCsrSortBigCap * 4);
-  constexpr size_t pool = sizeof(SearchPool) * (kSearchBlock / 32);
-  if (e == cudaSuccess) e = set((const void*)k_smooth_search<true>, pool);
-  if (e == cudaSuccess) e = set((const void*)k_smooth_search<false>, pool);
+  if (e == cudaSuccess) e = set((const void*)k_smooth_search<true, true>, kSearchSmem);
+  if (e == cudaSuccess) e = set((const void*)k_smooth_search<true, false>, kSearchSmem);
+  if (e == cudaSuccess) e = set((const void*)k_smooth_search<false, true>, kSearchSmem);
+  if (e == cudaSuccess) e = set((const void*)k_smooth_search<false, false>, kSearchSmem);
   return e;
 }
 

@@ -188,7 +188,8 @@ struct StepConst {
   int32_t qe_df;     // element shares are double-float pairs (the FP64 variants of arithmetic 2)
   int32_t stab_off[13];  // SMOOTH: offset of the subdivision table of valence N in DevBuf::stab, or -1
   uint32_t irr_first;   // first irregular internal face (SMOOTH: face index of DevBuf::icoef)
-  int32_t irr_levels;   // subdivision levels whose children's power forms are kept in DevBuf::icoef
+  int32_t irr_levels;   // subdivision levels whose children's power forms are kept in DevBuf::icoef: the first
+                        // ones and the last
   int32_t friction;  // 1 if mu_s or mu_d != 0
   int32_t pressure_base, pressure_dir;
   int32_t compat_zero_pressure;
@@ -279,7 +280,7 @@ struct DevBuf {
   double* lcoef;               // per original face with a regular patch: the limit surface's power form
                                // (SHL_LIMIT_NCOEF), made before each search from the current positions
   double* icoef;               // the same of the irregular faces' subdivision children: [face - irr_first]
-                               // [level - 1 < irr_levels][child]
+                               // [stored level < irr_levels][child]
   uint32_t* inv_perm;          // original -> internal face
   int32_t* fsm;                // per original face: valence | (position of the patch's first vertex) << 8
   double* stab;                // subdivision tables of the valences present

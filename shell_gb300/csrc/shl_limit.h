@@ -268,14 +268,28 @@ SHL_HD double shl_limit_child_point(const shl_limit_patch* pt, int n, int k, int
   return Q;
 }
 
+/* The child's power form: all three components in one pass over each row (in three
+ * passes, an irregular mesh's searches that make their own forms took 1.5 times as
+ * long). */
 SHL_HD void shl_limit_coeffs_child(const shl_limit_patch* pt, int n, int k, double P[15][3])
 {
+  const int np = pt->N + 6;
+  const double* T = pt->tab + (size_t)((n - 1) * 3 + k) * 12 * (size_t)np;
   SHL_UNROLL
   for (int m = 0; m < 15; ++m) P[m][0] = P[m][1] = P[m][2] = 0.0;
   SHL_UNROLL
-  for (int s = 0; s < 12; ++s)
-    shl_limit_add_point(P, s, shl_limit_child_point(pt, n, k, s, 0), shl_limit_child_point(pt, n, k, s, 1),
-                        shl_limit_child_point(pt, n, k, s, 2));
+  for (int s = 0; s < 12; ++s) {
+    double Q0 = 0.0, Q1 = 0.0, Q2 = 0.0;
+    for (int j = 0; j < np; ++j) {
+      const double t = T[s * np + j];
+      if (t == 0.0) continue;
+      const double* x = pt->base + 3 * (size_t)pt->ids[(size_t)j * pt->stride];
+      Q0 = SHL_FMA(t, x[0], Q0);
+      Q1 = SHL_FMA(t, x[1], Q1);
+      Q2 = SHL_FMA(t, x[2], Q2);
+    }
+    shl_limit_add_point(P, s, Q0, Q1, Q2);
+  }
   shl_limit_scale(P);
 }
 
