@@ -235,20 +235,34 @@ shl_status check_launch(const char* where) {
 
 
 
-// Makes the corrector-side linked-cell pass that fused steps may have left
-// pending, so the candidate list and du_sum are those of the unfused sequence
-// at this point (before the host reads or changes the state).
+// Makes the corrector-side linked-cell pass that fused steps have left pending
+// (h: the control block, read and refreshed), so the candidate list and du_sum are
+// those of the unfused sequence at this point (before the host reads or changes the
+// state).  A run that a problem ended gets the pass of its last step all the same.
+shl_status deferred_pass(shl_ctx* c, Ctl& h) {
+  const int32_t halted = h.halted;
+  if (halted) {
+    h.halted = 0;
+    SHL_TRY(ctl_put(c, h));
+  }
+  launch_rebuild_first(c->b, c->sc, c->stream);
+  launch_rebuild(c->b, c->sc, c->stream);
+  SHL_TRY(check_launch("deferred linked-cell pass"));
+  SHL_TRY(ctl_get(c, h));
+  if (halted) {
+    h.halted = halted;
+    SHL_TRY(ctl_put(c, h));
+  }
+  return SHL_OK;
+}
+
 shl_status flush_deferred_rebuild(shl_ctx* c) {
   if (!c->maybe_pending) return SHL_OK;
   c->maybe_pending = false;
   if (!c->sc.contact) return SHL_OK;
   Ctl h;
   SHL_TRY(ctl_get(c, h));
-  if (!h.rebuild_pending) return SHL_OK;
-  launch_rebuild_first(c->b, c->sc, c->stream);
-  launch_rebuild(c->b, c->sc, c->stream);
-  SHL_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return check_launch("deferred linked-cell pass");
+  return h.rebuild_pending ? deferred_pass(c, h) : SHL_OK;
 }
 
 // entry points that read the contact state or may change the step state
@@ -1453,12 +1467,7 @@ shl_status collect(shl_ctx* c, shl_step_report* report, const Ctl* fresh = nullp
   if (c->maybe_pending) {
     // a corrector-side linked-cell pass left pending by the last fused step
     c->maybe_pending = false;
-    if (c->sc.contact && h.rebuild_pending) {
-      launch_rebuild_first(c->b, c->sc, c->stream);
-      launch_rebuild(c->b, c->sc, c->stream);
-      SHL_TRY(check_launch("deferred linked-cell pass"));
-      SHL_TRY(ctl_get(c, h));
-    }
+    if (c->sc.contact && h.rebuild_pending) SHL_TRY(deferred_pass(c, h));
   }
   if (report) {
     std::memset(report, 0, sizeof(*report));

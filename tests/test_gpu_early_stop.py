@@ -86,3 +86,37 @@ def test_fields_of_the_last_step(cuda_ok, kind, last):
             assert d[k] == g[k], k
         else:
             assert np.array_equal(d[k], g[k]), k
+
+
+def test_list_after_a_problem(cuda_ok):
+    """The step that a problem ends may have made a linked-cell pass due: graph runs make it
+    when they report or the list is read, as direct launches make it at the end of the step."""
+    X, T = L.icosphere(3)
+    p = physics_params(cell_size_mult=cell_size_mult_for(X, T, 0.01), stop_on_problem=1)
+    u0 = _pressed(X, 3)
+    # the middle band set in motion: half the thickness in one step
+    v0 = np.zeros_like(X)
+    v0[np.abs(X[:, 0]) < 0.3, 2] = 60.0
+    out = []
+    for use_graph, read in ((False, False), (True, False), (True, True)):
+        g = L.Shell(X, T, p)
+        g.set_state(u0, v0.reshape(-1), np.zeros_like(u0))
+        g.rebuild_contacts()
+        if read:  # the list is read before the steps are collected
+            g.step_collect()  # the report starts here, as step() lets it
+            g.upload_pressure_table(np.zeros(N))
+            g.step_enqueue(N)
+            g.contact_state()
+            r, st = g.step_collect()
+        else:
+            r, st = g.step(N, np.zeros(N), use_graph=use_graph)
+        assert r.worst_problem == 2 and r.steps_done < N  # LARGE_DISP
+        c = g.contact_state()
+        one = [r.steps_done, r.n_rebuilds, r.du_sum, c["du_sum"], c["pairs"], c["stick"], _bits(c["origin"]), _bits(c["d2"])]
+        r, _ = g.step(2, np.zeros(2), use_graph=use_graph)
+        one += [r.steps_done, r.n_rebuilds] + [_bits(x) for x in g.get_state()]
+        out.append(one)
+        g.close()
+    assert out[0][1] >= 2  # the build, the predictor's pass, the corrector's
+    for k, (a, b, c) in enumerate(zip(*out)):
+        assert np.array_equal(a, b) and np.array_equal(a, c), k
