@@ -191,16 +191,50 @@ void split_to_soa(const Setup& S, std::vector<float>& out) {
     }
 }
 
-// the faces' split records as float pairs
-shl_status upload_split(shl_ctx* c) {
-  const std::vector<double>& r = c->S.split;
-  std::vector<float> t(2 * r.size());
-  for (size_t k = 0; k < r.size(); ++k) {
-    t[2 * k] = (float)r[k];
-    t[2 * k + 1] = (float)(r[k] - (double)t[2 * k]);
+// A device table made once, published when it is filled.
+template <class T>
+shl_status make_table(shl_ctx* c, T** table, const std::vector<T>& src) {
+  T* p = nullptr;
+  SHL_TRY(dev_alloc(c, &p, src.size()));
+  SHL_TRY(upload(c, p, src.data(), src.size()));
+  SHL_CUDA_TRY(cudaStreamSynchronize(c->stream));  // the source may be released
+  *table = p;
+  return SHL_OK;
+}
+
+// the regular faces' patch ids, face by face
+shl_status make_patch12(shl_ctx* c) {
+  if (c->b.patch12) return SHL_OK;
+  const Setup& S = c->S;
+  std::vector<int32_t> ids(12 * (size_t)S.groups[0].count);
+  for (uint32_t i = 0; i < S.groups[0].count; ++i)
+    for (int k = 0; k < 12; ++k) ids[12 * (size_t)i + k] = S.patch[(size_t)k * S.F + i];
+  return make_table(c, &c->b.patch12, ids);
+}
+
+// The constants that an FP64 variant's kernels read, if the context does not have
+// them yet: 464 bytes a face for the component-split kernels (records and patch ids),
+// 304 for the face-per-thread ones.  A context starts with those of its own
+// arithmetic; a forced variant or an FP32 context's FP64 residual may add others.
+shl_status need_fp64_constants(shl_ctx* c, int variant) {
+  const int pairs = kElemVariants[variant].pairs;
+  if (pairs == 2) {
+    SHL_TRY(make_patch12(c));
+    if (!c->b.face_df) {  // the split records as float pairs
+      const std::vector<double>& r = c->S.split;
+      std::vector<float> t(2 * r.size());
+      for (size_t k = 0; k < r.size(); ++k) {
+        t[2 * k] = (float)r[k];
+        t[2 * k + 1] = (float)(r[k] - (double)t[2 * k]);
+      }
+      SHL_TRY(make_table(c, &c->b.face_df, t));
+    }
   }
-  SHL_TRY(upload(c, c->b.face_df, t.data(), t.size()));
-  SHL_CUDA_TRY(cudaStreamSynchronize(c->stream));  // t is released here
+  if (pairs == 3 && !c->b.face_soa) {
+    std::vector<float> soa;
+    if (c->S.face_soa.empty()) split_to_soa(c->S, soa);
+    SHL_TRY(make_table(c, &c->b.face_soa, c->S.face_soa.empty() ? soa : c->S.face_soa));
+  }
   return SHL_OK;
 }
 
@@ -739,11 +773,7 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
     ALLOC(b.qe32, 3 * (size_t)S.n_slots_total);
     ALLOC(b.up32, (size_t)V);
     ALLOC(b.face32, (size_t)kFace32Stride * F);
-  } else {
-    ALLOC(b.face_df, (size_t)2 * kSplitStride * F);
-    if (params->shell_shell_contact == SHL_CONTACT_SMOOTH) ALLOC(b.face_soa, S.face_soa.size());
   }
-  ALLOC(b.patch12, 12 * (size_t)S.groups[0].count);
   ALLOC(b.qe, fp32 ? 1 : 3 * (size_t)S.n_slots_total);
   ALLOC(b.gather_ptr, V + 1);
   ALLOC(b.slot_pos, S.slot_pos.size());
@@ -755,7 +785,7 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
   ALLOC(b.perm, F);
   ALLOC(b.pscale, F);
   ALLOC(b.area, F); ALLOC(b.kG, F); ALLOC(b.kM, F); ALLOC(b.etens, F); ALLOC(b.ebend, F);
-  if (!params->adapt_dt_every) {  // pipelined steps
+  if (!params->adapt_dt_every && params->bulk_modulus == 0.0) {  // pipelined steps
     ALLOC(b.area_odd, F); ALLOC(b.kG_odd, F); ALLOC(b.kM_odd, F); ALLOC(b.etens_odd, F); ALLOC(b.ebend_odd, F);
   }
   // element launch: one block range per patch group
@@ -879,12 +909,7 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
   if ((st = upload(c, b.C, S.C.data(), nd)) != SHL_OK) return fail(st);
   if ((st = upload(c, b.face, S.face.data(), S.face.size())) != SHL_OK) return fail(st);
   if (fp32 && (st = upload(c, b.face32, S.face32.data(), S.face32.size())) != SHL_OK) return fail(st);
-  if (!fp32 && (st = upload_split(c)) != SHL_OK) return fail(st);
-  if (b.face_soa && (st = upload(c, b.face_soa, S.face_soa.data(), S.face_soa.size())) != SHL_OK) return fail(st);
-  std::vector<int32_t> patch12(12 * (size_t)S.groups[0].count);
-  for (uint32_t i = 0; i < S.groups[0].count; ++i)
-    for (int k = 0; k < 12; ++k) patch12[12 * (size_t)i + k] = S.patch[(size_t)k * F + i];
-  if (!patch12.empty() && (st = upload(c, b.patch12, patch12.data(), patch12.size())) != SHL_OK) return fail(st);
+  if (fp32 && (st = make_patch12(c)) != SHL_OK) return fail(st);
   if ((st = upload(c, b.patch, S.patch.data(), S.patch.size())) != SHL_OK) return fail(st);
   if ((st = upload(c, b.gather_ptr, S.gather_ptr.data(), S.gather_ptr.size())) != SHL_OK) return fail(st);
   if ((st = upload(c, b.slot_pos, S.slot_pos.data(), S.slot_pos.size())) != SHL_OK) return fail(st);
@@ -1007,6 +1032,7 @@ shl_status create_common(shl_ctx* c, const std::vector<double>& pscale_orig, shl
   sc.irr_first = irr_first;
   sc.irr_levels = irr_levels;
   c->var64 = default_var64(sc);
+  if (!fp32 && (st = need_fp64_constants(c, c->var64)) != SHL_OK) return fail(st);
   apply_variant(c);
   for (int k = 0; k < 13; ++k) sc.stab_off[k] = stab_off[k];
   sc.friction = (contact && (p.mu_s != 0 || p.mu_d != 0)) ? 1 : 0;
@@ -1936,14 +1962,7 @@ shl_status shl_residual(shl_ctx* c, double pressure, int flags, double* rel, dou
   }
   if (fp64 && ctx32) {  // the double-float FP64 path's shares and constants
     if (!c->qe64) SHL_TRY(dev_alloc(c, &c->qe64, 3 * (size_t)c->S.n_slots_total));
-    if (!c->b.face_df) {
-      SHL_TRY(dev_alloc(c, &c->b.face_df, 2 * c->S.split.size()));
-      SHL_TRY(upload_split(c));
-    }
-    if (c->sc.smooth && !c->b.face_soa) {
-      SHL_TRY(dev_alloc(c, &c->b.face_soa, c->S.face_soa.size()));
-      SHL_TRY(upload(c, c->b.face_soa, c->S.face_soa.data(), c->S.face_soa.size()));
-    }
+    SHL_TRY(need_fp64_constants(c, c->var64));
   }
   if (correct && !c->f32) SHL_TRY(dev_alloc(c, &c->f32, nd));
   if (correct && !c->b.fcorr) {
@@ -2191,14 +2210,7 @@ shl_status shl_set_element_variant(shl_ctx* c, int variant) {
     g_err = "element variant does not exist for this precision";
     return SHL_ERR_ARG;
   }
-  if (kElemVariants[variant].pairs == 3 && !c->b.face_soa) {
-    // the face-per-thread kernels read the constants row by row
-    std::vector<float> soa;
-    split_to_soa(c->S, soa);
-    SHL_TRY(dev_alloc(c, &c->b.face_soa, soa.size()));
-    SHL_TRY(upload(c, c->b.face_soa, soa.data(), soa.size()));
-    SHL_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  }
+  if (!c->sc.fp32) SHL_TRY(need_fp64_constants(c, variant));
   if (c->sc.fp32) c->var32 = variant; else c->var64 = variant;
   apply_variant(c);
   if (c->graph) cudaGraphExecDestroy(c->graph);
