@@ -381,8 +381,9 @@ constexpr uint32_t kWideFaces = 8192;
 // the cells lo..hi of a face, G lanes at a time: calls at(cell)
 template <int G, class Fn>
 __device__ __forceinline__ void walk_cells(const GridView& g, const int* lo, const int* hi, uint32_t sub, Fn at) {
-  const uint32_t total = shl_cells_covered(lo, hi);
-  for (uint32_t q = sub; q < total; q += G) at(g.base + shl_cells_at(q, lo, hi, g.ny, g.nz));
+  const int l[3] = {lo[0], lo[1], lo[2]}, h[3] = {hi[0], hi[1], hi[2]};  // at() stores: not to be read again
+  const uint32_t total = shl_cells_covered(l, h);
+  for (uint32_t q = sub; q < total; q += G) at(g.base + shl_cells_at(q, l, h, g.ny, g.nz));
 }
 
 // cell ranges (ShellSystem.C:1982-1983) and histogram of the faces (G = 1 or a

@@ -2441,11 +2441,16 @@ __global__ void __launch_bounds__(kBlock) k_correct_adapt(DevBuf b, StepConst sc
 }
 
 // ------------------------------------------------------ volume, end step --
+// ODD: the step's per-face fields are in the second set (kVolMeasureOdd).  Its own
+// instantiation: as a branch of the one kernel, whose end small shells wait for, it
+// took a 3,920-face shell in a cavity 1 % longer a step.
+template <bool ODD>
 __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, int mode) {
   Ctl* ctl = b.ctl;
   const bool end_step = mode == kVolEndStep;
   // a pipelined step was ended by its corrector, which may have stopped the run
-  if (mode >= kVolMeasure ? ctl->measure == 0 : inactive(ctl)) return;
+  const bool stopped = ODD && inactive(ctl);  // wanted at the end: its loads are beside the others
+  if (mode == kVolMeasure ? ctl->measure == 0 : inactive(ctl)) return;
   if (end_step && sc.adapt_every && !ctl->accept) {
     // a repeated attempt ends no step; only a step size below the machine
     // precision (SHL_SMALL_TIMESTEP) ends the run (ShellSystem.C:1110-1117)
@@ -2467,14 +2472,6 @@ __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, i
   double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   if (f < sc.F) {
     face_totals(b, f, v);
-    // a run that stopped with this step reads its fields from the first set
-    if (mode == kVolMeasureOdd && inactive(ctl)) {
-      b.area_odd[f] = b.area[f];
-      b.kG_odd[f] = b.kG[f];
-      b.kM_odd[f] = b.kM[f];
-      b.etens_odd[f] = b.etens[f];
-      b.ebend_odd[f] = b.ebend[f];
-    }
     const double* q0 = b.p + 3 * (size_t)b.tri[3 * (size_t)f];
     const double* q1 = b.p + 3 * (size_t)b.tri[3 * (size_t)f + 1];
     const double* q2 = b.p + 3 * (size_t)b.tri[3 * (size_t)f + 2];
@@ -2485,6 +2482,13 @@ __global__ void __launch_bounds__(kBlock) k_volume_end(DevBuf b, StepConst sc, i
   if (threadIdx.x == 0) {
     double* pp = b.partial_v + (size_t)blockIdx.x * 8;
     for (int k = 0; k < 6; ++k) pp[k] = v[k];
+  }
+  if (ODD && stopped && f < sc.F) {  // the fields are read from the first set
+    b.area_odd[f] = b.area[f];
+    b.kG_odd[f] = b.kG[f];
+    b.kM_odd[f] = b.kM[f];
+    b.etens_odd[f] = b.etens[f];
+    b.ebend_odd[f] = b.ebend[f];
   }
   if (!last_block(&ctl->cnt[4])) return;
   // the cavity's surface on a warp that has no column to sum, beside the sums
@@ -2751,7 +2755,10 @@ void launch_correct_adapt(const DevBuf& b, const StepConst& sc, cudaStream_t s, 
 }
 
 void launch_volume_end_step(const DevBuf& b, const StepConst& sc, int mode, cudaStream_t s) {
-  k_volume_end<<<nblk(sc.F), kBlock, 0, s>>>(b, sc, mode);
+  if (mode == kVolMeasureOdd)
+    k_volume_end<true><<<nblk(sc.F), kBlock, 0, s>>>(b, sc, kVolMeasure);
+  else
+    k_volume_end<false><<<nblk(sc.F), kBlock, 0, s>>>(b, sc, mode);
 }
 
 // ================================================================ no-alloc --
