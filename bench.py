@@ -73,22 +73,20 @@ STEP_BYTES_PER_FACE = 456
 # FP64 flops of one regular face in the element kernel (count of the
 # arithmetic in element_force<12>, fused multiply-add = 2)
 ELEM_FLOPS_PER_FACE = 1372
-# DRAM bytes (read + write) of one launch of the tuned element kernel (the
-# component-split kernel, 64 x 12) on the level-6 shell, from one ncu capture with
-# caches flushed (44.6 MB read, 0.7 MB written: the shares stay in L2)
-ELEM_TRAFFIC_LEVEL6 = 45.3e6
+# DRAM bytes (read + write; the shares stay in L2) and warp instructions
+# (smsp__inst_executed.sum) of one launch of each shape of the component-split
+# element kernel on the level-6 shell, one ncu capture each with caches flushed
+# (profiles/k_elements_split_and_gather.md); None for a shape that was not captured
+ELEM_TRAFFIC_LEVEL6 = {"fp64 128x5 split": 44.8e6, "fp64 64x8 split": 44.7e6, "fp64 64x12 split": 45.0e6}
+ELEM_WARP_INST_LEVEL6 = {"fp64 128x5 split": 22.93e6, "fp64 64x8 split": 22.86e6, "fp64 64x12 split": 23.19e6}
 # FP32 element path (the ensemble): about 300 algorithmic bytes per face-step with
-# FP32 per-face constants; DRAM bytes of one launch on the 256-shell ensemble and its
+# FP32 per-face constants; DRAM bytes of one launch on the 256-shell ensemble
 # (671.3 MB read, 407.9 MB written: the force shares do not fit in L2 at this size;
-# one ncu capture) and the FP32-pipe utilisation of the same arithmetic before its
-# constants came as records (a lower bound now)
+# one ncu capture) and the FMA pipe's share of active cycles (48 shells)
 ENS_BYTES_PER_FACE = 300
-ENS_ELEM_TRAFFIC = 1079.2e6
-ENS_ELEM_FP32_PIPE = 0.129
-# warp instructions of one element-kernel launch on the level-6 shell (ncu
-# smsp__inst_executed.sum of the same capture) and the issue peak: 4 schedulers
-# per SM, one warp instruction per cycle each
-ELEM_WARP_INST_LEVEL6 = 22.95e6
+ENS_ELEM_TRAFFIC = {"fp32 64x12": 1079.2e6}
+ENS_ELEM_FP32_PIPE = {"fp32 256x2": 0.165, "fp32 128x5": 0.176, "fp32 64x12": 0.180}
+# the issue peak: 4 schedulers per SM, one warp instruction per cycle each
 ISSUE_PER_SM_PER_CYCLE = 4
 
 
@@ -193,11 +191,11 @@ def time_ensemble(L, torch, K, W, flush):
             "dtype": "f32 forces, f64 state and contact gaps", "contact": "linear + friction, per-shell linked cells",
             "steps": K, "status": int(status), "n_pairs": int(n_pairs), "shell_rebuilds_total": int(nr0.sum()),
             "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
-                         "traffic": ENS_ELEM_TRAFFIC, "kernel": "k_elements32", "variant": elem_variant,
-                         "kernel_ms": elem_ms, "fp32_pipe_frac": ENS_ELEM_FP32_PIPE,
+                         "traffic": ENS_ELEM_TRAFFIC.get(elem_variant), "kernel": "k_elements32", "variant": elem_variant,
+                         "kernel_ms": elem_ms, "fp32_pipe_frac": ENS_ELEM_FP32_PIPE.get(elem_variant),
                          "algorithmic_bytes": "%d B per face-step x %d faces" % (ENS_BYTES_PER_FACE, F),
-                         "note": "the FP32 element kernel of the batched path, timed live; traffic and FP32-pipe "
-                                 "share from one ncu capture (the larger fraction, HBM, is the bound)"},
+                         "note": "the FP32 element kernel of the batched path, timed live; traffic and FMA-pipe "
+                                 "share of active cycles from ncu captures of the variant"},
             "contact_heavy": {"value": F * K / (ms_c * 1e-3), "ms_per_step": ms_c / K, "n_pairs": int(pairs_c),
                               "shell_rebuilds_in_timed_steps": int((nr2 - nr1).sum()),
                               "status": int(status_c),
@@ -749,6 +747,7 @@ def run_ours(args, rank, world, dist):
     clocks = clk.summary()
     sm_ghz = (clocks.get("sm_max_mhz") or 2070.0) / 1e3
     issue_peak = ISSUE_PER_SM_PER_CYCLE * 152 * sm_ghz  # G warp instructions / s
+    warp_inst = ELEM_WARP_INST_LEVEL6.get(elem_variant) if args.level == 6 else None
     if rank != 0:
         return
     cpu = None
@@ -776,17 +775,15 @@ def run_ours(args, rank, world, dist):
                        "kernel each way)"},
         "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm, "unit": "GB/s",
                      "frac": achieved_gbs / hbm,
-                     "traffic": ELEM_TRAFFIC_LEVEL6 if args.level == 6 else None,
-                     "traffic_note": "bytes per launch, ncu capture of the level-6 element kernel",
+                     "traffic": ELEM_TRAFFIC_LEVEL6.get(elem_variant) if args.level == 6 else None,
+                     "traffic_note": "bytes per launch, ncu capture of this variant at level 6",
                      "algorithmic_bytes": "%d B per face-step x %d faces" % (STEP_BYTES_PER_FACE, F),
                      "kernel": "k_elements", "variant": elem_variant,
                      "kernel_ms": elem_ms, "peak_source": hbm_src,
-                     "issue": {"warp_inst_per_launch": ELEM_WARP_INST_LEVEL6 if args.level == 6 else None,
-                               "achieved_ginst_s": (ELEM_WARP_INST_LEVEL6 / (elem_ms * 1e-3) / 1e9
-                                                    if args.level == 6 else None),
+                     "issue": {"warp_inst_per_launch": warp_inst,
+                               "achieved_ginst_s": warp_inst / (elem_ms * 1e-3) / 1e9 if warp_inst else None,
                                "peak_ginst_s": issue_peak,
-                               "frac": (ELEM_WARP_INST_LEVEL6 / (elem_ms * 1e-3) / 1e9 / issue_peak
-                                        if args.level == 6 else None),
+                               "frac": warp_inst / (elem_ms * 1e-3) / 1e9 / issue_peak if warp_inst else None,
                                "note": "instruction issue: the bound of the double-float element kernel "
                                        "(4 warp instructions per SM per cycle at the sampled max SM clock)"},
                      "fp64": {"achieved_tflops": achieved_tf, "peak_tflops": fp64_peak,

@@ -10,11 +10,12 @@
 // operations are one instruction instead of three, cross products and dot
 // products exchange neighbours' components by shuffles, and each row of the
 // stress resultants is one lane's.  The chain is a third as long and needs 96
-// registers, so that twice the warps share an SM.  Cold, in us: 1,280 faces
-// 59 -> 30, 81,920 faces 77 -> 56, 163,840 faces 132 -> 84 (warm, 8,820 faces
-// 34 -> 15).  Summing products in one accumulator, exact power-of-two weights and
-// sums made by one lane for all three took 163,840 faces from 84 to 72.  Bound by
-// FP32 issue at the large end (64 % of the slots) and by the chain at the small.
+// registers, so that twice the warps share an SM.  Cold, in us, against the thread
+// per face: 1,280 faces 59 -> 30, 81,920 faces 77 -> 47, 163,840 faces 132 -> 72
+// (warm, 8,820 faces 34 -> 15).  Of that, summing products in one accumulator, exact
+// power-of-two weights and sums made by one lane for all three are 84 -> 72 at
+// 163,840 faces.  Bound by FP32 issue at the large end (61-64 % of the slots) and by
+// the chain at the small.
 //
 // The mechanics are those of the relative-displacement form: no step subtracts
 // nearly equal quantities.
